@@ -526,6 +526,507 @@ __global__ void tfim_sample_kernel(const float* __restrict__ W, int n,
   }
 }
 
+// ---------------------------------------------------------------------------
+// Register form of the sampler, n <= 2048: one warp per shot, lane l owns the
+// nodes [l C, (l + 1) C) (C = ceil(n / 32) rounded up to a group) and keeps
+// their float64 weights in registers, in groups of SR_GS whose sums it also
+// keeps. A pick is then: the lanes' totals scanned over the warp, the owner of
+// the hit found by ballot, its node by halving (each decision is the owner's,
+// broadcast by a vote, so the branches are uniform and the registers' indices
+// known at compile time), and one pass over the groups that the picked row
+// touches - multiply and re-sum, never a running difference. The form above
+// moves every weight through shared memory three times per pick (its bound);
+// here a weight costs one predicated float64 multiply and one add, and the
+// bound is instruction issue. Picks multiply each weight by the same factors
+// in the same order as above, so the weights are the same numbers; only the
+// order of the sums differs.
+//
+// The rows come as tables built from W at the start of the call, in the
+// workspace (nothing is kept between calls): bit planes for weights in {0, +1,
+// -1}, else the float64 factor of every entry. Control words tell which form
+// the weights call for, so nothing is read back to the host: the kernels of the
+// other forms return at once. Times: see tfim_sample_impl.
+constexpr int SR_GS = 8;           // nodes per group
+constexpr int SR_MAX_N = 32 * 64;  // C <= 64
+
+// Sparse form (below): row slots
+constexpr int SP_DEG = 15;
+constexpr int SP_CODE_DEG = 7;
+
+struct __align__(16) SparseEntry {
+  double factor;
+  int col;    // the row's own node for an empty slot
+  int minus;  // weight -1
+};
+
+// Control words: some weight is -1; some weight is not in {0, +1, -1}; nonzero
+// weights; the largest number of them in a row.
+struct SampleCtl {
+  unsigned minus, other, count, degree;
+};
+
+// Tables of W's rows, a warp per row through shared memory:
+//  * planes +1, -1, nonzero (n * 32 * NW words each): row r, lane l: NW =
+//    ceil(C / 32) words of the lane's C nodes, lowest first;
+//  * table (nullable): factors (1 where the weight is 0), row r as C / 2 runs
+//    of 32 lanes x 2 nodes: lane l's nodes l C + 2 q and + 1 at (32 q + l) * 2,
+//    so a warp of the sampler reads a run as one contiguous 512 bytes;
+//  * slots (nullable): the first SP_DEG nonzero weights in column order.
+// One block sets the control words itself; more add to zeroed ones.
+__global__ void __launch_bounds__(1024) tfim_rows_kernel(const float* __restrict__ W, int n, int C, double base,
+                                 uint32_t* __restrict__ planes, double* __restrict__ table,
+                                 SparseEntry* __restrict__ slots, SampleCtl* __restrict__ ctl) {
+  extern __shared__ float rows_smem[];
+  __shared__ SampleCtl sc;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  const int NW = (C + 31) / 32, plane = n * 32 * NW;
+  float* buf = rows_smem + (size_t)wib * 32 * (C + 1);  // node v at v + v / C: lanes on distinct banks
+  const double lnb = log(base);
+  const double rep1 = exp(-lnb), repm1 = exp(lnb);
+  auto factor = [&](float w) {
+    return w == 0.0f ? 1.0 : w == 1.0f ? rep1 : w == -1.0f ? repm1 : repulsion_factor(lnb, w);
+  };
+  if (threadIdx.x == 0) sc = SampleCtl{0u, 0u, 0u, 0u};
+  __syncthreads();
+  unsigned minus_any = 0, other = 0, count = 0, degree = 0;
+  for (int r = blockIdx.x * wpb + wib; r < n; r += gridDim.x * wpb) {
+    const float* row = W + (size_t)r * n;
+    int at = 0;
+    for (int v = lane; v < 32 * C; v += 32) {
+      const float w = v < n ? __ldg(row + v) : 0.0f;
+      buf[v + v / C] = w;
+      const unsigned nz = __ballot_sync(0xFFFFFFFFu, w != 0.0f);
+      if (slots && w != 0.0f) {
+        const int e = at + __popc(nz & ((1u << lane) - 1u));
+        if (e < SP_DEG) slots[(size_t)r * SP_DEG + e] = SparseEntry{factor(w), v, w == -1.0f};
+      }
+      at += __popc(nz);
+    }
+    if (slots && lane >= at && lane < SP_DEG) slots[(size_t)r * SP_DEG + lane] = SparseEntry{1.0, r, 0};
+    degree = max(degree, (unsigned)at);
+    count += lane == 0 ? at : 0;
+    __syncwarp();
+    for (int q = 0; q < NW; ++q) {
+      uint32_t plus = 0, minus = 0, nz = 0;
+      for (int i = 0; i < min(32, C - 32 * q); ++i) {
+        const float w = buf[lane * (C + 1) + 32 * q + i];
+        if (w == 1.0f) plus |= 1u << i;
+        if (w == -1.0f) minus |= 1u << i;
+        if (w != 0.0f) nz |= 1u << i;
+      }
+      const int e = (r * 32 + lane) * NW + q;
+      planes[e] = plus;
+      planes[plane + e] = minus;
+      planes[2 * plane + e] = nz;
+      minus_any |= minus;
+      other |= nz & ~(plus | minus);
+    }
+    if (table)
+      for (int x = lane; x < 32 * C; x += 32) {
+        const int v = ((x >> 1) & 31) * C + 2 * (x >> 6) + (x & 1);
+        table[(size_t)r * (32 * C) + x] = factor(buf[v + v / C]);
+      }
+    __syncwarp();
+  }
+  if (minus_any) atomicOr(&sc.minus, 1u);
+  if (other) atomicOr(&sc.other, 1u);
+  if (count) atomicAdd(&sc.count, count);
+  if (lane == 0) atomicMax(&sc.degree, degree);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (gridDim.x == 1) {
+      *ctl = sc;
+    } else {
+      if (sc.minus) atomicOr(&ctl->minus, 1u);
+      if (sc.other) atomicOr(&ctl->other, 1u);
+      atomicAdd(&ctl->count, sc.count);
+      atomicMax(&ctl->degree, sc.degree);
+    }
+  }
+}
+
+// Which form the weights call for. codes / lists: the sparse forms are there
+// (chosen by n in tfim_sample_impl).
+enum SampleForm { SF_BITS, SF_TABLE, SF_LISTS, SF_CODES };
+__device__ __forceinline__ SampleForm sample_form(const SampleCtl& c, bool codes, bool lists) {
+  if (codes && !c.other && c.degree <= SP_CODE_DEG) return SF_CODES;
+  if (lists && c.degree <= SP_DEG) return SF_LISTS;
+  return c.other ? SF_TABLE : SF_BITS;
+}
+
+// w *= f where bit != 0. The jump makes it one predicated multiply; written as
+// a conditional it became a multiply and two selects (ER n = 1024, 32768
+// shots: 10.0 ms against 7.6 ms).
+__device__ __forceinline__ void mul_if(double& w, uint32_t bit, double f) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p bra SKIP;\n\tmul.rn.f64 %0, %0, %2;\n\tSKIP:\n\t}"
+      : "+d"(w)
+      : "r"(bit), "d"(f));
+}
+
+// Inclusive scan over the warp: a lane's sum with the lanes below it (the
+// shuffle's own predicate says whether there is one).
+__device__ __forceinline__ double warp_scan(double x) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 lo, hi;\n\t.reg .f64 y;\n\t"
+        "mov.b64 {lo, hi}, %0;\n\t"
+        "shfl.sync.up.b32 lo, lo, %1, 0, 0xFFFFFFFF;\n\t"
+        "shfl.sync.up.b32 hi|p, hi, %1, 0, 0xFFFFFFFF;\n\t"
+        "mov.b64 y, {lo, hi};\n\t"
+        "@!p bra SKIP;\n\tadd.rn.f64 %0, %0, y;\n\tSKIP:\n\t}"
+        : "+d"(x)
+        : "r"(o));
+  return x;
+}
+
+// w[LO] + ... + w[LO + N - 1], pairwise
+template <int LO, int N, int C>
+__device__ __forceinline__ double tree_sum(const double (&w)[C]) {
+  if constexpr (N == 1) {
+    return w[LO];
+  } else {
+    return tree_sum<LO, (N + 1) / 2, C>(w) + tree_sum<LO + (N + 1) / 2, N / 2, C>(w);
+  }
+}
+
+// The owner's node holding q among w[LO .. LO + N): its index, and its weight
+// becomes zero. Groups are passed over by their sums, then the nodes of one.
+template <int LO, int N, int C>
+__device__ __forceinline__ int pick_node(double (&w)[C], const double (&sum)[C / SR_GS], double q, int owner,
+                                         int lane) {
+  if constexpr (N == 1) {
+    if (lane == owner) w[LO] = 0.0;
+    return LO;
+  } else {
+    constexpr int H = N > SR_GS ? (N / SR_GS + 1) / 2 * SR_GS : N / 2;
+    double m;
+    if constexpr (N > SR_GS) {
+      m = tree_sum<LO / SR_GS, H / SR_GS, C / SR_GS>(sum);
+    } else {
+      m = tree_sum<LO, H, C>(w);
+    }
+    const unsigned below = __ballot_sync(0xFFFFFFFFu, q < m);
+    if ((below >> owner) & 1u) return pick_node<LO, H, C>(w, sum, q, owner, lane);
+    return pick_node<LO + H, N - H, C>(w, sum, q - m, owner, lane);
+  }
+}
+
+// Resident blocks of 64 threads per SM, by measurement (ER and complete graphs
+// of 32 C nodes): the latency of a pick wants warps, the weights want 2 C
+// registers; a few spilled words cost less than a block, and the factor loads
+// of TABLE need more registers in flight.
+constexpr int sr_blocks(int C, bool table) {
+  return C >= 56 ? 6 : C >= 48 ? (table ? 6 : 7) : C >= 40 ? 8 : C >= 32 ? 10 : C >= 24 ? (table ? 10 : 14) : (table && C >= 16 ? 14 : 16);
+}
+
+template <int C, bool TABLE>
+__global__ void __launch_bounds__(64, sr_blocks(C, TABLE))
+    tfim_sample_reg_kernel(int n, const double* __restrict__ cum, int ncum, double base, int repel, uint64_t seed,
+                           uint64_t round, int shots, uint32_t* __restrict__ theta_out,
+                           const uint32_t* __restrict__ planes, const double* __restrict__ table,
+                           const SampleCtl* __restrict__ ctl, bool codes, bool lists) {
+  constexpr int NG = C / SR_GS, NW = (C + 31) / 32;
+  const SampleCtl ct = *ctl;
+  if (sample_form(ct, codes, lists) != (TABLE ? SF_TABLE : SF_BITS)) return;
+  const bool has_minus = ct.minus != 0;
+  // factors of sparse rows are loaded one by one where the weight is not zero
+  const bool sparse = (long long)ct.count * 4 < (long long)n * n;
+  const int lane = threadIdx.x & 31;
+  const int n32 = (n + 31) >> 5;
+  const double lnb = log(base);
+  const double rep1 = exp(-lnb), repm1 = exp(lnb);
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const int plane = n * 32 * NW;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < shots; s += warps) {
+    const uint64_t key = mix64(seed ^ mix64(round * 0x632BE59BD9B4E019ull + (uint64_t)s));
+    // uniform(seed, round, s, draw) with the shot's part worked out once
+    auto draw = [&](int d) {
+      const uint64_t h = mix64(key ^ ((uint64_t)d * 0xD1B54A32D192ED03ull));
+      return (double)(h >> 11) * (1.0 / 9007199254740992.0);
+    };
+    const int m = sample_mag(cum, ncum, draw(0));
+    int node = s % n;
+    uint32_t* out = theta_out + (size_t)s * n32;
+    if (m == 1) {
+      for (int w = lane; w < n32; w += 32) out[w] = (w == (node >> 5)) ? (1u << (node & 31)) : 0u;
+      continue;
+    }
+    // all ones but the first pick
+    double w[C], sum[NG];
+#pragma unroll
+    for (int i = 0; i < C; ++i) w[i] = (lane * C + i < n && lane * C + i != node) ? 1.0 : 0.0;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) sum[g] = 0.0;
+    int slot = node % C;
+    double us = 0.0;  // lane l: the draw of pick j with j % 32 == l
+    // picks after the first node: m - 1 for m >= 2, one for m == 0
+    const int picks = (m == 0) ? 1 : m - 1;
+#pragma unroll 1
+    for (int j = 1; j <= picks; ++j) {
+      if (j == 1 || (j & 31) == 0) us = draw((j & ~31) + lane);
+      // update_repulsion_choice (maxcut_tfim.py:37-45) for the node picked
+      // last, and the sums of the groups that changed (all of them at first)
+      uint32_t nz[NW], any[NW];
+#pragma unroll
+      for (int q = 0; q < NW; ++q) {
+        nz[q] = repel ? __ldg(planes + (TABLE ? 2 * plane : 0) + (node * 32 + lane) * NW + q) : 0u;
+        any[q] = j == 1 ? 0xFFFFFFFFu
+                        : __reduce_or_sync(0xFFFFFFFFu, nz[q]) | ((slot >> 5) == q ? 1u << (slot & 31) : 0u);
+      }
+      if constexpr (TABLE) {
+        const double* row = table + (size_t)node * (32 * C) + 2 * lane;
+        if (!repel) {
+#pragma unroll
+          for (int g = 0; g < NG; ++g) sum[g] = tree_sum<0, SR_GS, SR_GS>(*reinterpret_cast<double(*)[SR_GS]>(&w[SR_GS * g]));
+        } else if (sparse) {
+#pragma unroll
+          for (int g = 0; g < NG; ++g) {
+            const uint32_t b = nz[SR_GS * g / 32] >> ((SR_GS * g) & 31);
+            if (((any[SR_GS * g / 32] >> ((SR_GS * g) & 31)) & 0xFFu) == 0u) continue;
+            double f[SR_GS];
+#pragma unroll
+            for (int i = 0; i < SR_GS; ++i) {
+              f[i] = 1.0;
+              if ((b >> i) & 1u) f[i] = __ldg(row + 64 * ((SR_GS * g + i) >> 1) + (i & 1));
+            }
+#pragma unroll
+            for (int i = 0; i < SR_GS; ++i) w[SR_GS * g + i] *= f[i];
+            sum[g] = tree_sum<0, SR_GS, SR_GS>(*reinterpret_cast<double(*)[SR_GS]>(&w[SR_GS * g]));
+          }
+        } else {
+#pragma unroll
+          for (int g = 0; g < NG; ++g) {
+#pragma unroll
+            for (int i = 0; i < SR_GS; i += 2) {
+              const double2 f = __ldg(reinterpret_cast<const double2*>(row + 32 * (SR_GS * g + i)));
+              w[SR_GS * g + i] *= f.x;
+              w[SR_GS * g + i + 1] *= f.y;
+            }
+            sum[g] = tree_sum<0, SR_GS, SR_GS>(*reinterpret_cast<double(*)[SR_GS]>(&w[SR_GS * g]));
+          }
+        }
+      } else {
+        uint32_t mm[NW], anym[NW];
+#pragma unroll
+        for (int q = 0; q < NW; ++q) {
+          mm[q] = anym[q] = 0u;
+          if (has_minus) {
+            mm[q] = repel ? __ldg(planes + plane + (node * 32 + lane) * NW + q) : 0u;
+            anym[q] = __reduce_or_sync(0xFFFFFFFFu, mm[q]);
+          }
+        }
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          const int q = SR_GS * g / 32, sh = (SR_GS * g) & 31;
+          if ((((any[q] | anym[q]) >> sh) & 0xFFu) == 0u) continue;
+#pragma unroll
+          for (int i = 0; i < SR_GS; ++i) mul_if(w[SR_GS * g + i], nz[q] & (1u << (sh + i)), rep1);
+          if ((anym[q] >> sh) & 0xFFu) {
+#pragma unroll
+            for (int i = 0; i < SR_GS; ++i) mul_if(w[SR_GS * g + i], mm[q] & (1u << (sh + i)), repm1);
+          }
+          sum[g] = tree_sum<0, SR_GS, SR_GS>(*reinterpret_cast<double(*)[SR_GS]>(&w[SR_GS * g]));
+        }
+      }
+      // bit_pick (util:711-724): p = sum(weights) * u, the first node whose
+      // running sum is above p (node 0 when none is)
+      const double loc = tree_sum<0, NG, NG>(sum);
+      const double incl = warp_scan(loc);
+      const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
+      const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
+      if (hit) {
+        const int owner = __ffs(hit) - 1;
+        slot = pick_node<0, C, C>(w, sum, p - (incl - loc), owner, lane);
+        node = owner * C + slot;
+      } else {
+        if (lane == 0) w[0] = 0.0;
+        slot = node = 0;
+      }
+    }
+    // selection mask: weights == 0 (picked, or underflowed to zero); lane l
+    // holds bits [l C, l C + C)
+    uint64_t bits = 0;
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+      if (lane * C + i < n && w[i] == 0.0) bits |= 1ull << i;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) {
+      // word 32 q + lane: bits from the lane holding its first node on
+      const int word = 32 * q + lane, src = 32 * word / C, off = 32 * word - src * C;
+      uint64_t v = 0;
+#pragma unroll
+      for (int t = 0; t * C < 32 + C; ++t) {
+        const uint64_t o = __shfl_sync(0xFFFFFFFFu, bits, (src + t) & 31);
+        const int at = t * C - off;  // position of that lane's first bit in the word
+        if (src + t < 32 && at < 32) v |= at >= 0 ? o << at : o >> -at;
+      }
+      if (word < n32) out[word] = (uint32_t)v;
+    }
+  }
+}
+
+// Sparse form, n <= 2048 and at most SP_DEG nonzero weights in any row: one
+// warp per shot with the weights in shared memory and the sums of groups of 32
+// nodes beside them. A pick scans the groups' sums and then one group's weights;
+// an update touches the picked node's neighbours, one row slot per lane, and
+// sums their groups anew, so a pick costs O(degree) groups instead of n weights.
+// The chain of a pick (a row load, the groups' sums, two scans) is latency, so
+// what counts is how many shots an SM holds: float64 weights leave 13 at n =
+// 2048. Where every weight is +-1 and no row has more than SP_CODE_DEG (CODES),
+// a weight is one of 2^(SP_CODE_DEG + 1) products of factors in the order of the
+// picks, so a byte names it - a leading 1, then a bit per factor; 0 for a picked
+// node - and a table holds the products, multiplied in that order.
+// Shared memory of one shot: the groups' sums, then the weights or codes of
+// 1024 GP nodes. CODES blocks hold the table of products before them.
+constexpr int SP_TABLE = 1 << (SP_CODE_DEG + 1);
+constexpr int sp_shot_bytes(int GP, bool codes) { return 32 * GP * 8 + 1024 * GP * (codes ? 1 : 8); }
+constexpr int sp_warps(bool codes) { return codes ? 4 : 1; }  // shots per block
+
+template <int GP, bool CODES>
+__global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
+    tfim_sample_sparse_kernel(int n, const double* __restrict__ cum, int ncum, double base, int repel, uint64_t seed,
+                              uint64_t round, int shots, uint32_t* __restrict__ theta_out,
+                              const SparseEntry* __restrict__ slots, const SampleCtl* __restrict__ ctl, bool codes,
+                              bool lists) {
+  const SampleCtl ct = *ctl;
+  if (sample_form(ct, codes, lists) != (CODES ? SF_CODES : SF_LISTS)) return;
+  const int deg = (int)ct.degree;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31;
+  const int n32 = (n + 31) >> 5;  // groups of 32 nodes, and words of a packed row
+  double* table = reinterpret_cast<double*>(smem);
+  double* gsum = reinterpret_cast<double*>(smem + (CODES ? SP_TABLE * 8 : 0) +
+                                           (threadIdx.x >> 5) * sp_shot_bytes(GP, CODES));
+  double* w = gsum + 32 * GP;
+  uint8_t* code = reinterpret_cast<uint8_t*>(w);
+  if constexpr (CODES) {
+    const double lnb = log(base);
+    const double rep1 = exp(-lnb), repm1 = exp(lnb);
+    for (int c = threadIdx.x; c < SP_TABLE; c += blockDim.x) {
+      double x = c ? 1.0 : 0.0;
+      for (int b = 30 - __clz(c | 1); b >= 0; --b) x *= ((c >> b) & 1) ? repm1 : rep1;
+      table[c] = x;
+    }
+    __syncthreads();
+  }
+  auto weight = [&](int v) -> double {
+    if constexpr (CODES) {
+      return table[code[v]];
+    } else {
+      return w[v];
+    }
+  };
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < shots; s += warps) {
+    const uint64_t key = mix64(seed ^ mix64(round * 0x632BE59BD9B4E019ull + (uint64_t)s));
+    auto draw = [&](int d) {
+      const uint64_t h = mix64(key ^ ((uint64_t)d * 0xD1B54A32D192ED03ull));
+      return (double)(h >> 11) * (1.0 / 9007199254740992.0);
+    };
+    const int m = sample_mag(cum, ncum, draw(0));
+    int node = s % n;
+    uint32_t* out = theta_out + (size_t)s * n32;
+    if (m == 1) {
+      for (int q = lane; q < n32; q += 32) out[q] = (q == (node >> 5)) ? (1u << (node & 31)) : 0u;
+      continue;
+    }
+    // all ones but the first pick
+    for (int v = lane; v < 1024 * GP; v += 32) {
+      const bool one = v < n && v != node;
+      if constexpr (CODES) {
+        code[v] = one ? 1 : 0;
+      } else {
+        w[v] = one ? 1.0 : 0.0;
+      }
+    }
+    for (int g = lane; g < 32 * GP; g += 32) {
+      const int left = n - 32 * g;
+      gsum[g] = (double)(left >= 32 ? 32 : left > 0 ? left : 0);
+    }
+    __syncwarp();
+    double us = 0.0;  // lane l: the draw of pick j with j % 32 == l
+    const int picks = (m == 0) ? 1 : m - 1;
+#pragma unroll 1
+    for (int j = 1; j <= picks; ++j) {
+      if (j == 1 || (j & 31) == 0) us = draw((j & ~31) + lane);
+      // update_repulsion_choice (maxcut_tfim.py:37-45) for the node picked
+      // last: lane l its row's slot l (lanes from deg on: the node itself, whose
+      // group changed too)
+      int col = node;
+      if (repel && lane < deg) {
+        const SparseEntry e = slots[(size_t)node * SP_DEG + lane];
+        col = e.col;
+        if constexpr (CODES) {
+          const int c = code[col];
+          // (a row picked twice, which takes a draw that no prefix is above,
+          // could lengthen a full code: left as it is)
+          if (c && c < SP_TABLE / 2 && col != node) code[col] = (uint8_t)(2 * c + e.minus);
+        } else {
+          if (col != node) w[col] *= e.factor;
+        }
+      }
+      __syncwarp();
+      // the touched groups' sums, four at a time by eight lanes each
+      const int last = repel ? deg : 0;
+#pragma unroll 1
+      for (int c = 0; c <= last; c += 4) {
+        const int g = __shfl_sync(0xFFFFFFFFu, col, min(c + (lane >> 3), last)) >> 5;
+        double x;
+        if constexpr (CODES) {
+          const uint32_t c4 = *reinterpret_cast<const uint32_t*>(code + 32 * g + 4 * (lane & 7));
+          x = (table[c4 & 255u] + table[(c4 >> 8) & 255u]) + (table[(c4 >> 16) & 255u] + table[c4 >> 24]);
+        } else {
+          const double* wg = w + 32 * g + (lane & 7);
+          x = (wg[0] + wg[8]) + (wg[16] + wg[24]);
+        }
+        x += __shfl_xor_sync(0xFFFFFFFFu, x, 1);
+        x += __shfl_xor_sync(0xFFFFFFFFu, x, 2);
+        x += __shfl_xor_sync(0xFFFFFFFFu, x, 4);
+        if ((lane & 7) == 0) gsum[g] = x;
+      }
+      __syncwarp();
+      // bit_pick (util:711-724): lane l holds the groups GP l .. GP l + GP - 1
+      double gs[GP];
+#pragma unroll
+      for (int i = 0; i < GP; ++i) gs[i] = gsum[GP * lane + i];
+      const double loc = tree_sum<0, GP, GP>(gs);
+      const double incl = warp_scan(loc);
+      const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
+      const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
+      node = 0;  // no prefix above p
+      if (hit) {
+        const int owner = __ffs(hit) - 1;
+        double q = p - (incl - loc);
+        int g = GP * owner;
+        if constexpr (GP == 2) {
+          const bool up = !(q < gs[0]);
+          if (up) q -= gs[0];
+          g += (__ballot_sync(0xFFFFFFFFu, up) >> owner) & 1u;
+        }
+        q = __shfl_sync(0xFFFFFFFFu, q, owner);
+        const unsigned h2 = __ballot_sync(0xFFFFFFFFu, q < warp_scan(weight(32 * g + lane)));
+        node = 32 * g + (h2 ? __ffs(h2) - 1 : 0);
+      }
+      if (lane == 0) {
+        if constexpr (CODES) {
+          code[node] = 0;
+        } else {
+          w[node] = 0.0;
+        }
+      }
+      __syncwarp();
+    }
+    // selection mask: weights == 0 (picked, or underflowed to zero)
+    for (int g = 0; g < n32; ++g) {
+      const unsigned b = __ballot_sync(0xFFFFFFFFu, 32 * g + lane < n && weight(32 * g + lane) == 0.0);
+      if (lane == 0) out[g] = b;
+    }
+    __syncwarp();
+  }
+}
+
 // Nonzero counts of W's rows (warp per row).
 __global__ void tfim_adj_count_kernel(const float* __restrict__ W, int n, long long* __restrict__ count) {
   const int lane = threadIdx.x & 31;
@@ -654,6 +1155,8 @@ pqi_status pqi_tfim_cdf(const double* J_eff, const unsigned int* degrees, int n,
 
 size_t pqi_tfim_sample_workspace_bytes(int n) {
   const int C = (n + 31) / 32;
+  // weight tables of the warps (nodes past shared memory), or the register
+  // form's row tables (n <= 2048: at most 34 MB, within the former)
   return (size_t)148 * 16 * kWtsPitch * C * sizeof(double) + 4096;
 }
 
@@ -664,9 +1167,78 @@ static pqi_status tfim_sample_impl(const float* W, int n, const double* cum, dou
   // W is read only without row lists (the dense row scan)
   PQI_CHECK_ARG((W || adj_ptr) && cum && theta_out && n >= 3 && shots > 0);
   cudaStream_t s = as_stream(stream);
+  const int repel = fabs(1.0 - repulsion_base) <= kEps ? 0 : 1;
+  // Up to 2048 nodes with W at hand (and the workspace that
+  // pqi_tfim_sample_workspace_bytes names): weights in registers, or the sparse
+  // forms - codes from 257 nodes (reg 512: 0.72 ms against 0.80 for 8192 shots),
+  // lists from 1025, where the registers hold two warps a scheduler (3-regular
+  // 2048: 9.3 ms against 17.0). Milliseconds per round, shared-memory form -> now:
+  // ER 1024, 32768 shots 34.9 -> 6.4; ER 2048, 8192 39.7 -> 7.5; complete float
+  // 1024, 8192 16.4 -> 2.9; complete float 2000, 4096 49.3 -> 6.9; 3-regular 2048,
+  // 16384 19.2 -> 4.3; G(1500, 0.1) float, 8192 12.2 -> 9.4; ER 64, 4096 0.19 -> 0.09.
+  if (W && n <= SR_MAX_N) {
+    const int RC = ((n + 31) / 32 + SR_GS - 1) / SR_GS * SR_GS, NW = (RC + 31) / 32;
+    // codes need factors and their products well inside float64's range
+    const bool codes = n > 256 && repulsion_base > 1e-40 && repulsion_base < 1e40;
+    const bool lists = n > 1024;
+    Workspace ws(workspace, workspace_bytes);
+    SampleCtl* ctl = ws.take<SampleCtl>(1);
+    uint32_t* planes = ws.take<uint32_t>((size_t)3 * n * 32 * NW);
+    double* table = ws.take<double>((size_t)n * 32 * RC);
+    SparseEntry* slots = codes || lists ? ws.take<SparseEntry>((size_t)n * SP_DEG) : nullptr;
+    if (ctl && planes && table && (slots || !(codes || lists))) {
+      // small graphs: one block, which needs no zeroed control words
+      const int rb = n <= 256 ? 1 : std::min((n + 3) / 4, 148 * 4), rw = n <= 256 ? 32 : 4;
+      if (rb > 1) PQI_TRY(cudaMemsetAsync(ctl, 0, sizeof(SampleCtl), s));
+      tfim_rows_kernel<<<rb, 32 * rw, (size_t)rw * 32 * (RC + 1) * sizeof(float), s>>>(W, n, RC, repulsion_base,
+                                                                                     planes, table, slots, ctl);
+      PQI_LAUNCHED("tfim_rows_kernel");
+      auto sparse = [&](auto kern, int GP, bool cd) -> pqi_status {
+        const int wb = sp_warps(cd);
+        const size_t sm = (size_t)wb * sp_shot_bytes(GP, cd) + (cd ? SP_TABLE * sizeof(double) : 0);
+        int per_sm = 1;
+        PQI_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        PQI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wb, sm));
+        const int g = (int)std::min<long long>(((long long)shots + wb - 1) / wb, 148ll * std::max(1, per_sm));
+        kern<<<g, 32 * wb, sm, s>>>(n, cum, n - 1, repulsion_base, repel, seed, round, shots, theta_out, slots, ctl,
+                                    codes, lists);
+        PQI_LAUNCHED("tfim_sample_sparse_kernel");
+        return PQI_OK;
+      };
+      auto dense = [&](auto kern, int blocks) -> pqi_status {
+        const int g = (int)std::min<long long>(((long long)shots + 1) / 2, 148ll * blocks);
+        kern<<<g, 64, 0, s>>>(n, cum, n - 1, repulsion_base, repel, seed, round, shots, theta_out, planes, table,
+                              ctl, codes, lists);
+        PQI_LAUNCHED("tfim_sample_reg_kernel");
+        return PQI_OK;
+      };
+      pqi_status rc = PQI_OK;
+      if (codes)
+        rc = n <= 1024 ? sparse(tfim_sample_sparse_kernel<1, true>, 1, true)
+                       : sparse(tfim_sample_sparse_kernel<2, true>, 2, true);
+      if (rc == PQI_OK && lists) rc = sparse(tfim_sample_sparse_kernel<2, false>, 2, false);
+      if (rc != PQI_OK) return rc;
+#define PQI_SR_CASE(C_)                                                         \
+  case C_:                                                                     \
+    rc = dense(tfim_sample_reg_kernel<C_, false>, sr_blocks(C_, false));        \
+    if (rc == PQI_OK) rc = dense(tfim_sample_reg_kernel<C_, true>, sr_blocks(C_, true)); \
+    break
+      switch (RC) {
+        PQI_SR_CASE(8);
+        PQI_SR_CASE(16);
+        PQI_SR_CASE(24);
+        PQI_SR_CASE(32);
+        PQI_SR_CASE(40);
+        PQI_SR_CASE(48);
+        PQI_SR_CASE(56);
+        PQI_SR_CASE(64);
+      }
+#undef PQI_SR_CASE
+      return rc;
+    }
+  }
   const int C = (n + 31) / 32;
   const size_t per_warp = (size_t)C * kWtsPitch * sizeof(double);
-  const int repel = fabs(1.0 - repulsion_base) <= kEps ? 0 : 1;
   int wpb = 4;
   size_t smem = per_warp * wpb;
   int use_smem = 1;

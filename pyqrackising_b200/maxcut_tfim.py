@@ -228,16 +228,17 @@ def row_lists(dg: D.DeviceGraph):
 def sample_batch(dg: D.DeviceGraph, cum, shots: int, repulsion_base: float, seed: int, round_: int, out=None,
                  lists="auto"):
     """One round of shot_loop (maxcut_tfim.py:139-145) on the device: `shots`
-    candidates as packed words [shots, ceil(n/32)]. Graphs with few nonzero
-    weights per row use row lists for the repulsion updates (`lists`: "auto",
-    or False for the row scan; both give the same draws)."""
+    candidates as packed words [shots, ceil(n/32)]. Graphs of more than 2048
+    nodes with few nonzero weights per row use row lists for the repulsion
+    updates (`lists`: "auto", or False for the row scan; both give the same draws)."""
     n = dg.n
     lib = _lib.load()
     if out is None:
         out = torch.empty(shots * dg.n32 + 1, dtype=torch.int32, device=dg.device)
         out[-1] = 0  # spare word (single-row 64-bit view), never written by the sampler
     ws = dg.ws.get(lib.pqi_tfim_sample_workspace_bytes(n))
-    rl = row_lists(dg) if lists == "auto" else None
+    # (up to 2048 nodes the dense matrix's call builds the row tables it needs itself)
+    rl = row_lists(dg) if lists == "auto" and not (n <= 2048 and hasattr(dg, "W")) else None
     if rl is not None:
         _lib.call(
             "pqi_tfim_sample_adj",
