@@ -5,9 +5,13 @@
 // Both keep each state's gain vector on chip and update it in O(n) per
 // accepted flip (g_v -= 2 x_v x_k W_kv, g_k = -g_k) instead of recomputing an
 // O(n) row sum for every candidate flip as the reference does.
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <type_traits>
 
 #include "pqi_common.cuh"
+#include "pqi_tc.cuh"
 
 namespace pqi {
 
@@ -176,65 +180,208 @@ __global__ void __launch_bounds__(256) gray_kernel(
   }
 }
 
-// Single CTA: repeat (select best single flip under the reference geometry,
+// ---------------------------------------------------------------------------
+// Descent: repeat (select the best single flip under the reference geometry,
 // flip it if its value is > 0) until none improves or max_flips is reached.
-template <typename WT>
-__global__ void __launch_bounds__(1024) descent_kernel(
-    const WT* __restrict__ Wp, int ld, int n, uint32_t* __restrict__ theta,
-    double* __restrict__ g64, int spin, SelGeom geo, int max_flips, int gains_in_smem,
-    double* __restrict__ energy_sum, int* __restrict__ flips, int* __restrict__ trace,
-    int* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ uint64_t scratch[32];
-  const int n32 = (n + 31) >> 5;
-  uint32_t* bits = reinterpret_cast<uint32_t*>(smem);
-  double* g = gains_in_smem
-                  ? reinterpret_cast<double*>(smem + (((size_t)n32 * 4 + 15) & ~size_t(15)))
-                  : g64;
-  for (int q = threadIdx.x; q < n32; q += blockDim.x) bits[q] = theta[q];
-  if (gains_in_smem)
-    for (int v = threadIdx.x; v < n; v += blockDim.x) g[v] = g64[v];
-  __syncthreads();
+//
+// The chain of a flip - row load, update, selection over all n nodes - is
+// serial, so the kernel is bound by its latency; a thread keeps the gains, bits
+// and tie priorities of 4 NG nodes in registers and the selection goes through
+// as few synchronisations as the size allows:
+//  * one warp (n <= 512): two redux steps, no barrier;
+//  * one CTA: each warp's best through shared memory, one barrier;
+//  * a cluster (CL): every warp sends its best to every CTA with st.async,
+//    counted on that CTA's mbarrier, and every warp waits for all of them and
+//    reduces them itself: one exchange, no CTA barrier. Two slot arrays and
+//    mbarriers alternate; a warp sends flip f + 2 only after all warps have
+//    read flip f (each sends f + 1 after that), so a slot is not overwritten
+//    while it is read.
+// While the row of the flipped node loads, the rows of new candidates - the next
+// flips are mostly among the warps' bests - are pulled into L2. Times: see pqi_single_descent.
+constexpr int DC_SLOTS = 256;  // warps of the largest launch: 16 CTAs x 512 threads
+
+struct __align__(16) DescentBest {
+  uint32_t hi;    // ordered float value (0: none selectable)
+  uint32_t lo;    // tie priority, larger first; 0: never selected
+  uint32_t node;  // node << 1 | its bit
+  uint32_t pad;
+};
+
+// The best of the warp's lanes, in every lane (priorities are unique).
+__device__ __forceinline__ DescentBest warp_best(const DescentBest& b) {
+  DescentBest r;
+  r.hi = __reduce_max_sync(0xFFFFFFFFu, b.hi);
+  r.lo = __reduce_max_sync(0xFFFFFFFFu, b.hi == r.hi ? b.lo : 0u);
+  const unsigned src = __ballot_sync(0xFFFFFFFFu, b.hi == r.hi && b.lo == r.lo);
+  r.node = __shfl_sync(0xFFFFFFFFu, b.node, __ffs(src) - 1);
+  r.pad = 0u;
+  return r;
+}
+
+__device__ __forceinline__ void better(DescentBest& b, const DescentBest& o) {
+  if (o.hi > b.hi || (o.hi == b.hi && o.lo > b.lo)) b = o;
+}
+
+template <typename WT, int NG, bool CL>
+__global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp, int ld, int n,
+                                                      uint32_t* __restrict__ theta, double* __restrict__ g64,
+                                                      int spin, SelGeom geo, int max_flips,
+                                                      double* __restrict__ energy_sum, int* __restrict__ flips,
+                                                      int* __restrict__ trace, int* __restrict__ status) {
+  namespace cg = cooperative_groups;
+  __shared__ DescentBest slots[2][DC_SLOTS];
+  __shared__ __align__(8) uint64_t bar[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = blockDim.x, nwarps = T >> 5;
+  int C = 1, rank = 0;
+  if constexpr (CL) {
+    C = (int)cg::this_cluster().num_blocks();
+    rank = (int)cg::this_cluster().block_rank();
+    if (threadIdx.x == 0) {
+      tc::mbar_init(&bar[0], 1);
+      tc::mbar_init(&bar[1], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cg::this_cluster().sync();
+  }
+  const int nslots = C * nwarps;
+  const int v0 = 4 * (rank * NG * T + (int)threadIdx.x);  // group j starts at v0 + 4 T j
+  double g[4 * NG];
+  uint32_t lo[4 * NG], xm = 0;
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    const int v = v0 + 4 * T * j;
+    if (v < ((n + 31) & ~31)) xm |= ((theta[v >> 5] >> (v & 31)) & 15u) << (4 * j);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool in = v + i < n;
+      g[4 * j + i] = in ? g64[v + i] : 0.0;
+      lo[4 * j + i] = in ? (uint32_t)sel_key(0.0f, (uint64_t)(v + i), geo) : 0u;
+    }
+  }
+  const int slice = 4 * rank * NG * T;  // this CTA's first node
+  const uint32_t slice_bytes = slice < ld ? (uint32_t)(min(4 * NG * T, ld - slice) * (int)sizeof(WT)) : 0u;
+  uint32_t seen = 0xFFFFFFFFu;
   double esum = 0.0;
   int cnt = 0, st = PQI_OK;
-  while (true) {
-    // a value below the thread's best so far cannot give a larger key: the
-    // key (and its divisions) only for candidates that reach it
-    uint64_t best = 0;
+  for (int f = 0;; ++f) {
+    // the thread's best, as floats (a -0 below a +0 does not matter here: only
+    // values above 0 are taken); NaN compares false throughout
     float bv = -INFINITY;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      float v = (float)g[k];
+    uint32_t bl = 0u, be = 0u;
+#pragma unroll
+    for (int e = 0; e < 4 * NG; ++e) {
+      float v = (float)g[e];
       if (spin) v *= 2.0f;
-      if (v >= bv) {
-        const uint64_t kk = sel_key(v, (uint64_t)k, geo);
-        if (kk > best) {
-          best = kk;
-          bv = v;
-        }
+      if (lo[e] != 0u && (v > bv || (v == bv && lo[e] > bl))) {
+        bv = v;
+        bl = lo[e];
+        be = (uint32_t)(v0 + 4 * T * (e >> 2) + (e & 3)) << 1 | ((xm >> e) & 1u);
       }
     }
-    best = block_max_u64(best, scratch);
-    float val;
-    int64_t idx;
-    sel_decode(best, geo, &val, &idx);
+    DescentBest b{bl ? ord_f32(bv) : 0u, bl, be, 0u};
+    b = warp_best(b);
+    const int par = f & 1;
+    if constexpr (CL) {
+      if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(nslots * sizeof(DescentBest)));
+      if (lane < C) {
+        uint32_t raddr, rbar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                     : "=r"(raddr)
+                     : "r"(tc::smem_u32(&slots[par][rank * nwarps + warp])), "r"(lane));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[par])), "r"(lane));
+        asm volatile(
+            "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
+            "l"((uint64_t)b.lo << 32 | b.hi), "l"((uint64_t)b.node), "r"(rbar)
+            : "memory");
+      }
+      if (!tc::mbar_wait_spin(&bar[par], (uint32_t)(f >> 1) & 1u)) {
+        st = PQI_ECUDA;  // a peer stopped sending
+        break;
+      }
+    } else if (nwarps > 1) {
+      if (lane == 0) slots[par][warp] = b;
+      __syncthreads();
+    }
+    if (CL || nwarps > 1) {
+      DescentBest c{0u, 0u, 0u, 0u};
+      for (int q = lane; q < nslots; q += 32) better(c, slots[par][q]);
+      b = warp_best(c);
+    }
+    const float val = b.lo ? unord_f32(b.hi) : -INFINITY;
     if (!(val > 0.0f)) break;
     if (cnt >= max_flips) {
       st = PQI_ETIMEOUT;
       break;
     }
     esum += (double)val;
-    if (threadIdx.x == 0 && trace) trace[cnt] = (int)idx;
+    const int k = (int)(b.node >> 1);
+    const uint32_t xk = b.node & 1u;
+    if (rank == 0 && threadIdx.x == 0 && trace) trace[cnt] = k;
     ++cnt;
-    block_flip<double, WT, uint32_t, 8>(g, bits, Wp, ld, n, (int)idx);
+    const WT* __restrict__ row = Wp + (size_t)k * ld;
+    WT w[4 * NG];
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+      const int v = v0 + 4 * T * j;
+      if (v < n) {  // (rows are zero padded to a multiple of 128)
+        if constexpr (sizeof(WT) == 4) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(row + v));
+          w[4 * j] = t.x; w[4 * j + 1] = t.y; w[4 * j + 2] = t.z; w[4 * j + 3] = t.w;
+        } else {
+          const char4 t = __ldg(reinterpret_cast<const char4*>(row + v));
+          w[4 * j] = t.x; w[4 * j + 1] = t.y; w[4 * j + 2] = t.z; w[4 * j + 3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[4 * j + i] = (WT)0;
+      }
+    }
+    if constexpr (CL) {
+      // This CTA's slice of the rows of new candidates (a warp's best that was
+      // not its best before), into L2: a hint. Warp w looks after warp w of
+      // every CTA, one per lane.
+      if (lane < C) {
+        const uint32_t node = slots[par][lane * nwarps + warp].node >> 1;
+        if (node != seen && slice_bytes > 0u) {
+          seen = node;
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Wp + (size_t)node * ld + slice),
+                       "r"(slice_bytes)
+                       : "memory");
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4 * NG; ++e) {
+      const int v = v0 + 4 * T * (e >> 2) + (e & 3);
+      const double w2 = 2.0 * (double)w[e];
+      if (v == k) {
+        g[e] = -g[e];
+        xm ^= 1u << e;
+      } else {
+        g[e] += ((xm >> e) & 1u) == xk ? -w2 : w2;
+      }
+    }
   }
-  for (int q = threadIdx.x; q < n32; q += blockDim.x) theta[q] = bits[q];
-  if (gains_in_smem)
-    for (int v = threadIdx.x; v < n; v += blockDim.x) g64[v] = g[v];
-  if (threadIdx.x == 0) {
+  // eight lanes assemble one word of 32 nodes
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    const int v = v0 + 4 * T * j;
+    uint32_t wd = ((xm >> (4 * j)) & 15u) << (4 * (lane & 7));
+    wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 1);
+    wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 2);
+    wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 4);
+    if ((lane & 7) == 0 && v < n) theta[v >> 5] = wd;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (v + i < n) g64[v + i] = g[4 * j + i];
+  }
+  if (rank == 0 && threadIdx.x == 0) {
     *energy_sum = esum;
     *flips = cnt;
-    if (status) *status = st;
+    *status = st;
   }
+  // (no CTA leaves while another may still send to it)
+  if constexpr (CL) cg::this_cluster().sync();
 }
 
 static size_t gray_smem_bytes(int n, size_t gain_bytes) {
@@ -243,6 +390,35 @@ static size_t gray_smem_bytes(int n, size_t gain_bytes) {
 }
 
 static constexpr size_t kMaxDynSmem = 200 * 1024;
+
+// Largest graph that descends in one CTA (512 threads of four nodes): at 2048
+// nodes 0.95 us per flip against 1.22 with a cluster, at 4096 (two groups per
+// thread) 1.32 against 1.17.
+constexpr int kDescentCta = 2048;  // 512 * 4 at most
+
+// CTAs of a descent's cluster: 16 where the device can place them.
+static int descent_cluster() {
+  static const int size = [] {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(512);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    const void* k = (const void*)descent_kernel<float, 16, true>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      return 8;
+    }
+    return 16;
+  }();
+  return size;
+}
 
 }  // namespace pqi
 
@@ -311,27 +487,62 @@ pqi_status pqi_single_descent(const pqi_weights* w, uint32_t* theta, double* gai
   int* status = ws.take<int>(1);
   PQI_CHECK_ARG(status);
   cudaStream_t s = as_stream(stream);
-  const size_t bits_bytes = (((size_t)((n + 31) >> 5) * 4 + 15) & ~size_t(15));
-  size_t smem = bits_bytes + (size_t)n * 8;
-  int in_smem = 1;
-  if (smem > kMaxDynSmem) {
-    smem = bits_bytes;
-    in_smem = 0;
-  }
-  PQI_CHECK_ARG(smem <= kMaxDynSmem);
-  if (w->kind == PQI_W_I8) {
-    PQI_TRY(cudaFuncSetAttribute(descent_kernel<int8_t>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    descent_kernel<int8_t><<<1, 1024, smem, s>>>(w->W_i8, w->ld, n, theta, gains64,
-                                                 is_spin_glass, geo, max_flips, in_smem,
-                                                 energy_sum, flips, trace, status);
+  // Threads of 4 NG nodes: one warp up to 128 nodes, one CTA up to kDescentCta,
+  // else a cluster. Microseconds per flip, one CTA with the gains in shared
+  // memory and the tie rule's divisions per node -> now: complete float graphs
+  // of 300 nodes 2.8 -> 1.1, 1000 3.9 -> 0.90, 2048 4.5 -> 0.95, 4096 5.6 -> 1.10,
+  // 8192 8.2 -> 1.35 (a whole descent 38.4 -> 6.3 ms), 16384 13.9 -> 1.52.
+  const int groups = (n + 3) / 4;
+  int C = 1, T = 32, NG = 1;
+  auto shape = [&](int c, int tmax) {
+    const int per = (groups + c - 1) / c;
+    C = c;
+    T = std::min(tmax, (per + 31) / 32 * 32);
+    const int ng = (per + T - 1) / T;
+    NG = ng <= 1 ? 1 : ng <= 2 ? 2 : ng <= 4 ? 4 : ng <= 8 ? 8 : ng <= 16 ? 16 : 0;
+  };
+  if (n <= 128) {
+    shape(1, 32);
+  } else if (n <= kDescentCta) {
+    shape(1, 512);
   } else {
-    PQI_TRY(cudaFuncSetAttribute(descent_kernel<float>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    descent_kernel<float><<<1, 1024, smem, s>>>(w->W_f32z, w->ld, n, theta, gains64,
-                                                is_spin_glass, geo, max_flips, in_smem, energy_sum,
-                                                flips, trace, status);
+    const int c = descent_cluster();
+    for (int tmax = 128; tmax <= 512; tmax *= 2) {  // fewest groups per thread first
+      shape(c, tmax);
+      if (NG == 1) break;
+    }
   }
+  PQI_CHECK_ARG(NG > 0);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.stream = s;
+  auto launch = [&](auto kern, auto wp) -> pqi_status {
+    if (C > 1) {
+      PQI_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      attr[0].val.clusterDim.x = C;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+    }
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(T);
+    PQI_TRY(cudaLaunchKernelEx(&cfg, kern, wp, w->ld, n, theta, gains64, is_spin_glass, geo, max_flips, energy_sum,
+                               flips, trace, status));
+    return PQI_OK;
+  };
+  auto pick = [&](auto wp) -> pqi_status {
+    typedef typename std::remove_const<typename std::remove_pointer<decltype(wp)>::type>::type WT;
+    if (C == 1)
+      return launch(descent_kernel<WT, 1, false>, wp);  // (512 threads of four nodes cover kDescentCta)
+    return NG == 1   ? launch(descent_kernel<WT, 1, true>, wp)
+           : NG == 2 ? launch(descent_kernel<WT, 2, true>, wp)
+           : NG == 4 ? launch(descent_kernel<WT, 4, true>, wp)
+           : NG == 8 ? launch(descent_kernel<WT, 8, true>, wp)
+                     : launch(descent_kernel<WT, 16, true>, wp);  // (past the dense matrices that fit)
+  };
+  const pqi_status rc = w->kind == PQI_W_I8 ? pick((const int8_t*)w->W_i8) : pick((const float*)w->W_f32z);
+  if (rc != PQI_OK) return rc;
   PQI_LAUNCHED("descent_kernel");
   int hst = 0;
   PQI_TRY(cudaMemcpyAsync(&hst, status, sizeof(int), cudaMemcpyDeviceToHost, s));
