@@ -25,56 +25,8 @@ struct GainOf<int8_t> {
   typedef int type;
 };
 
-template <typename W64>
-__device__ __forceinline__ int bit_of(const W64* bits, int v);
-
-template <>
-__device__ __forceinline__ int bit_of<uint64_t>(const uint64_t* bits, int v) {
+__device__ __forceinline__ int bit_of(const uint64_t* bits, int v) {
   return (int)((bits[v >> 6] >> (v & 63)) & 1ull);
-}
-template <>
-__device__ __forceinline__ int bit_of<uint32_t>(const uint32_t* bits, int v) {
-  return (int)((bits[v >> 5] >> (v & 31)) & 1u);
-}
-
-// Flip node k of the block's state: every thread updates its slice of the
-// gains, then one thread toggles the bit. Must be reached by all threads of
-// the block with the same k. Caller guarantees a barrier after its own reads
-// of g[k] / bits.
-template <typename GT, typename WT, typename W64, int CH = 16>
-__device__ __forceinline__ void block_flip(GT* g, W64* bits, const WT* __restrict__ Wp, int ld,
-                                           int n, int k) {
-  const int xk = bit_of<W64>(bits, k);
-  const WT* __restrict__ row = Wp + (size_t)k * ld;
-  __syncthreads();
-  // row read in chunks of CH per thread, loads issued before the gains change
-  for (int base = threadIdx.x; base < n; base += CH * blockDim.x) {
-    WT w[CH];
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      const int v = base + i * blockDim.x;
-      w[i] = v < n ? __ldg(row + v) : (WT)0;
-    }
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {
-      const int v = base + i * blockDim.x;
-      if (v < n) {
-        if (v == k) {
-          g[v] = -g[v];
-        } else {
-          const GT w2 = (GT)2 * (GT)w[i];
-          g[v] += (bit_of<W64>(bits, v) == xk) ? -w2 : w2;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    constexpr int kShift = sizeof(W64) == 8 ? 6 : 5;
-    constexpr int kMask = sizeof(W64) == 8 ? 63 : 31;
-    bits[k >> kShift] ^= (W64)1 << (k & kMask);
-  }
-  __syncthreads();
 }
 
 template <typename GT>
@@ -88,10 +40,24 @@ __device__ __forceinline__ int from_f64<int>(double v) {
   return (int)llrint(v);
 }
 
-// One CTA per seed (grid-stride). Dynamic smem: 64-bit state words, then the
-// gains (unless g_global is given: then CTA b uses g_global + b*n).
+// One CTA per seed (grid-stride). Dynamic smem: 64-bit state words, one 32-bit
+// word per 64-node block of which of its first 32 nodes have a gain > 0, then
+// the gains (unless g_global is given: then CTA b uses g_global + b*n).
+//
+// The walk visits iterations i = s + m S < iters_bound in order and in each the
+// nodes ctz(i + 1) + 64 b, b ascending, and flips those with a gain > 0 (i + 1
+// < 2^31, so only the first 31 nodes of a block are ever visited). Flips are
+// few from a local optimum, so the walk does not test position by position:
+// between flips the set of positive gains is fixed, and an iteration can be
+// passed over when no block has a positive node of its class c = ctz(i + 1).
+// `any` is the OR of the blocks' words; a warp tests 32 iterations per step
+// against it, then finds the block within the first that has one. Every flip
+// refreshes the words by ballot as it updates the gains. All warps walk alike
+// (identical ballots), so only flips need barriers. Times: see pqi_gray.
+constexpr int kGrayThreads = 512;
+
 template <typename WT>
-__global__ void __launch_bounds__(256) gray_kernel(
+__global__ void __launch_bounds__(kGrayThreads) gray_kernel(
     const WT* __restrict__ Wp, int ld, int n, const uint64_t* __restrict__ theta64,
     const double* __restrict__ base_g, int spin, long long iters_bound, int S,
     uint64_t* __restrict__ theta_out, float* __restrict__ energy_out,
@@ -100,13 +66,58 @@ __global__ void __launch_bounds__(256) gray_kernel(
   extern __shared__ __align__(16) unsigned char smem[];
   const int blocks = (n + 63) >> 6;
   uint64_t* bits = reinterpret_cast<uint64_t*>(smem);
+  uint32_t* pos = reinterpret_cast<uint32_t*>(bits + blocks);
   GT* g = g_global ? g_global + (size_t)blockIdx.x * n
-                   : reinterpret_cast<GT*>(smem + (((size_t)blocks * 8 + 15) & ~size_t(15)));
+                   : reinterpret_cast<GT*>(smem + (((size_t)blocks * 12 + 15) & ~size_t(15)));
   const int lane = threadIdx.x & 31;
+
+  // Flip node k: every thread updates its gains and the words of positive
+  // gains, then one thread toggles the bit (read again only after the next
+  // flip's first barrier). Reached by all threads with the same k.
+  auto flip = [&](int k) {
+    __syncthreads();  // every warp has read the gains and words of its choice; the last toggle is done
+    const int xk = bit_of(bits, k);
+    const WT* __restrict__ row = Wp + (size_t)k * ld;
+    constexpr int CH = 16;  // loads in flight per thread
+    for (int base = threadIdx.x; base < 64 * blocks; base += CH * kGrayThreads) {
+      WT w[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int v = base + i * kGrayThreads;
+        w[i] = v < n ? __ldg(row + v) : (WT)0;
+      }
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int v = base + i * kGrayThreads;
+        if (v - lane >= 64 * blocks) break;  // (the warp's 32 nodes are past the last block)
+        bool up = false;
+        if (v < n) {
+          GT y = g[v];
+          if (v == k) {
+            y = -y;
+          } else {
+            const GT w2 = (GT)2 * (GT)w[i];
+            y += (bit_of(bits, v) == xk) ? -w2 : w2;
+          }
+          g[v] = y;
+          up = y > (GT)0;
+        }
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, up);
+        if (lane == 0 && !(v & 32)) pos[v >> 6] = m;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) bits[k >> 6] ^= 1ull << (k & 63);
+  };
 
   for (int s = blockIdx.x; s < S; s += gridDim.x) {
     for (int q = threadIdx.x; q < blocks; q += blockDim.x) bits[q] = theta64[q];
-    for (int v = threadIdx.x; v < n; v += blockDim.x) g[v] = from_f64<GT>(base_g[v]);
+    for (int v = threadIdx.x; v < 64 * blocks; v += blockDim.x) {
+      const GT y = v < n ? from_f64<GT>(base_g[v]) : (GT)0;
+      if (v < n) g[v] = y;
+      const unsigned m = __ballot_sync(0xFFFFFFFFu, v < n && y > (GT)0);
+      if (lane == 0 && !(v & 32)) pos[v >> 6] = m;
+    }
     __syncthreads();
 
     // Seed mask of work-item s (kernels.cl:915-926): seed bit 63-b flips node
@@ -133,46 +144,59 @@ __global__ void __launch_bounds__(256) gray_kernel(
         const int node = ((w0 + q) << 6) + p;
         if (node < n) {
           E += (double)g[node];
-          block_flip<GT, WT, uint64_t>(g, bits, Wp, ld, n, node);
+          flip(node);
         } else if (node < (blocks << 6)) {
           // padding bit of the last word: no energy, kept for the output words
           __syncthreads();
           if (threadIdx.x == 0) bits[node >> 6] ^= 1ull << (node & 63);
-          __syncthreads();
         }
       }
     }
 
-    // Gray walk: positions p = m*blocks + b for i = s + m*S < iters_bound; the
-    // candidate node is ctz(i+1) + 64b; a flip is kept iff its gain is > 0. All
-    // warps scan the same 32 positions (identical ballots, no barrier) and the
-    // block applies the first accepted flip together.
+    auto any_class = [&]() {
+      uint32_t a = 0;
+      for (int b = lane; b < blocks; b += 32) a |= pos[b];
+      return __reduce_or_sync(0xFFFFFFFFu, a);
+    };
     const long long Pm = iters_bound > s ? (iters_bound - 1 - s) / S + 1 : 0;
-    const long long P = Pm * blocks;
-    long long p0 = 0;
-    while (p0 < P) {
-      const long long p = p0 + lane;
-      int k = -1;
-      bool pos = false;
-      if (p < P) {
-        const long long mm = p / blocks;
-        const int b = (int)(p - mm * blocks);
-        const long long i = (long long)s + mm * S;
-        k = (__ffsll(i + 1) - 1) + (b << 6);
-        if (k < n) pos = g[k] > (GT)0;
-      }
-      const unsigned bal = __ballot_sync(0xFFFFFFFFu, pos);
+    long long mi = 0;  // iteration, and its first block still to visit
+    int b0 = 0;
+    uint32_t any = any_class();
+    while (mi < Pm) {
+      const long long mm = mi + lane;
+      const int c = __ffsll((long long)s + mm * S + 1) - 1;
+      const unsigned bal = __ballot_sync(0xFFFFFFFFu, mm < Pm && c < 32 && ((any >> c) & 1u));
       if (!bal) {
-        p0 += 32;
+        mi += 32;
+        b0 = 0;
         continue;
       }
       const int f = __ffs(bal) - 1;
-      const int kk = __shfl_sync(0xFFFFFFFFu, k, f);
-      E += (double)g[kk];
-      block_flip<GT, WT, uint64_t>(g, bits, Wp, ld, n, kk);
-      p0 += f + 1;
+      if (f > 0) b0 = 0;
+      mi += f;
+      const int cc = __shfl_sync(0xFFFFFFFFu, c, f);
+      unsigned hit = 0;
+      for (; b0 < blocks; b0 += 32) {
+        hit = __ballot_sync(0xFFFFFFFFu, b0 + lane < blocks && ((pos[b0 + lane] >> cc) & 1u));
+        if (hit) break;
+      }
+      if (!hit) {
+        ++mi;
+        b0 = 0;
+        continue;
+      }
+      b0 += __ffs(hit) - 1;
+      const int k = cc + (b0 << 6);
+      E += (double)g[k];
+      flip(k);
+      any = any_class();
+      if (++b0 == blocks) {
+        ++mi;
+        b0 = 0;
+      }
     }
 
+    __syncthreads();  // the last toggle
     for (int q = threadIdx.x; q < blocks; q += blockDim.x)
       theta_out[(size_t)s * blocks + q] = bits[q];
     if (threadIdx.x == 0) energy_out[s] = (float)(spin ? E : E / 2.0);
@@ -386,10 +410,10 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
 
 static size_t gray_smem_bytes(int n, size_t gain_bytes) {
   const int blocks = (n + 63) >> 6;
-  return (((size_t)blocks * 8 + 15) & ~size_t(15)) + (size_t)n * gain_bytes;
+  return (((size_t)blocks * 12 + 15) & ~size_t(15)) + (size_t)n * gain_bytes;
 }
 
-static constexpr size_t kMaxDynSmem = 200 * 1024;
+static constexpr size_t kMaxGraySmem = 208 * 1024;
 
 // Largest graph that descends in one CTA (512 threads of four nodes): at 2048
 // nodes 0.95 us per flip against 1.22 with a cluster, at 4096 (two groups per
@@ -426,6 +450,9 @@ using namespace pqi;
 
 extern "C" {
 
+// 148 seeds, n^2 iterations in all, from a local optimum (microseconds, testing
+// 32 positions per step -> now): complete float graphs of 1000 nodes 49 -> 39,
+// 4096 464 -> 62, 8192 3282 -> 85, 24000 80750 -> 223; ER 2048 113 -> 56.
 pqi_status pqi_gray(const pqi_weights* w, const uint64_t* theta64, const double* gains64,
                     int is_spin_glass, int iters_bound, int seeds, uint64_t* theta_out,
                     float* energy_out, void* workspace, size_t workspace_bytes, void* stream) {
@@ -446,11 +473,10 @@ pqi_status pqi_gray(const pqi_weights* w, const uint64_t* theta64, const double*
   size_t smem = gray_smem_bytes(n, gbytes);
   int grid = seeds;
   void* gglob = nullptr;
-  if (smem > kMaxDynSmem) {
+  if (smem > kMaxGraySmem) {
     // gains in global memory, one n-vector per CTA
-    const int blocks = (n + 63) >> 6;
-    smem = (size_t)blocks * 8;
-    PQI_CHECK_ARG(smem <= kMaxDynSmem);
+    smem = gray_smem_bytes(n, 0);
+    PQI_CHECK_ARG(smem <= kMaxGraySmem);
     const size_t avail = (ws.size > ws.used + 256) ? (ws.size - ws.used - 256) : 0;
     const long long ctas = (long long)(avail / ((size_t)n * gbytes));
     PQI_CHECK_ARG(ctas >= 1);
@@ -461,13 +487,13 @@ pqi_status pqi_gray(const pqi_weights* w, const uint64_t* theta64, const double*
   if (i8) {
     PQI_TRY(cudaFuncSetAttribute(gray_kernel<int8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-    gray_kernel<int8_t><<<grid, 256, smem, s>>>(w->W_i8, w->ld, n, theta64, gains64,
+    gray_kernel<int8_t><<<grid, kGrayThreads, smem, s>>>(w->W_i8, w->ld, n, theta64, gains64,
                                                 is_spin_glass, iters_bound, seeds, theta_out,
                                                 energy_out, static_cast<int*>(gglob));
   } else {
     PQI_TRY(cudaFuncSetAttribute(gray_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-    gray_kernel<float><<<grid, 256, smem, s>>>(w->W_f32z, w->ld, n, theta64, gains64,
+    gray_kernel<float><<<grid, kGrayThreads, smem, s>>>(w->W_f32z, w->ld, n, theta64, gains64,
                                                is_spin_glass, iters_bound, seeds, theta_out,
                                                energy_out, static_cast<double*>(gglob));
   }
