@@ -952,6 +952,7 @@ size_t pqi_workspace_bytes(int n, long count) {
   size_t b = 1 << 16;                                   // scalars, keys, stats
   b += cnt_pad * ld * 4;                                // expanded +-1 operand (bf16 x2 worst case)
   b += ((size_t)ld / 64 + 2) * (size_t)count * 8;       // per-tile partial scores
+  b += (ld + 256) * 4 * 256;                            // masked diagonal tiles of the scoring (four planes)
   b += (size_t)count * 4 + 256;                         // per-candidate energies
   b += (size_t)n * 8 * 2 + 512;                         // base gains (f64) and f32 copy
   const size_t tiles = (size_t)((n + 31) / 32) * ((n + 31) / 32);

@@ -81,6 +81,10 @@ constexpr int PF_BYTES = PF * 128 * 16;  // 12 KB
 constexpr int SMEM_BYTES_FUSED = STAGES * STAGE_BYTES + PF_BYTES + 1024;
 static_assert(SMEM_BYTES_FUSED <= 227 * 1024, "fused ring fits");
 
+// Wait for the kernel before this one (a no-op unless launched as its
+// programmatic dependent).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Persistent scoring kernel: CTA c handles the contiguous tiles
@@ -124,7 +128,8 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
                     const __grid_constant__ CUtensorMap map_b0,
                     const __grid_constant__ CUtensorMap map_b1,
                     const __grid_constant__ CUtensorMap map_b2,
-                    const __grid_constant__ CUtensorMap map_b3, int planes, double qscale,
+                    const __grid_constant__ CUtensorMap map_b3,
+                    const __grid_constant__ CUtensorMap map_d, int tri, int planes, double qscale,
                     int n, int shots,
                     const uint32_t* __restrict__ theta, int n32, double upper_sum, int spin,
                     SelGeom geo, double* __restrict__ qpart, float* __restrict__ energies,
@@ -155,18 +160,36 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
   const int ntn = (n + BN - 1) / BN;
   const int ntm = (shots + BM - 1) / BM;       // 128-candidate blocks (finish bookkeeping)
   const int ntu = (shots + UM - 1) / UM;       // tile rows
-  const int ntiles = ntn * ntu;
-  // each unit walks one contiguous chunk of tiles (candidate-block major), so
-  // most blocks are finished by one unit with q kept in registers
-  const int t_begin = (int)(((long long)unit * ntiles) / units);
-  const int t_end = (int)(((long long)(unit + 1) * ntiles) / units);
   const int kb_per_pass = kInt8 ? (n + BK_BYTES - 1) / BK_BYTES : (n + 63) / 64;
+  // K blocks of node tile tn's pass: all of K, or (tri) those up to its own end
+  auto tile_kb = [&](int tn) { return tri ? min(2 * tn + 2, kb_per_pass) : kb_per_pass; };
+  // each unit walks one contiguous chunk of tiles (candidate-block major), so
+  // most blocks are finished by one unit with q kept in registers; chunks are
+  // cut at the tile boundaries nearest to equal numbers of K blocks
+  auto cut = [&](int u) {
+    const long long per = tri ? (long long)ntn * (ntn - 1) + kb_per_pass : (long long)ntn * kb_per_pass;
+    const long long at = (long long)u * ntu * per / units;
+    const int blk = (int)(at / per), rem = (int)(at - blk * per);
+    int tn = 0;  // last tile starting at or before rem
+    if (tri) {
+      tn = (int)sqrtf((float)rem);
+      while (tn > 0 && tn * (tn + 1) > rem) --tn;
+      while (tn + 1 < ntn && (tn + 1) * (tn + 2) <= rem) ++tn;
+      tn = min(tn, ntn - 1);
+      const int start = tn * (tn + 1);
+      if (2 * (rem - start) > tile_kb(tn)) ++tn;
+    } else {
+      tn = (2 * rem + kb_per_pass) / (2 * kb_per_pass);
+    }
+    return blk * ntn + tn;
+  };
+  const int t_begin = cut(unit), t_end = cut(unit + 1);
   // int8 operands: `planes` K passes, each its own accumulation (planes = 4:
   // the digit planes of float weights, combined exactly in the epilogue);
   // bf16: the hi and lo passes accumulate into one accumulator
-  const int upt = kInt8 ? planes : 1;                       // accumulations per tile
-  const int spu = kInt8 ? kb_per_pass : 2 * kb_per_pass;    // stages per accumulation
-  const int kblocks = upt * spu;                            // stages per tile
+  const int upt = kInt8 ? planes : 1;      // accumulations per tile
+  const int ppu = kInt8 ? 1 : 2;           // passes per accumulation
+  const int drows = ntn * BN;              // rows of one plane of the diagonal tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) {
@@ -207,10 +230,12 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
 
   if (warp == TMA_WARP) {
     if (lane == 0) {
+      pdl_wait();  // the expansion pass's operand and diagonal tiles
       uint32_t it = 0;
       bool ok = true;
       for (int t = t_begin; t < t_end && ok; ++t) {
         const int m0 = (t / ntn) * UM + rank * BM, n0 = (t % ntn) * BN + rank * (BN / 2);
+        const int tn = t % ntn, kbt = tile_kb(tn), kblocks = upt * ppu * kbt;
         int kp = 0, pass = 0;  // K block within its pass, pass (plane, or hi / lo)
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % NST;
@@ -222,7 +247,13 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
           const int kk = kInt8 ? kp * BK_BYTES : kp * 64;
           const CUtensorMap* mb =
               pass == 0 ? &map_b0 : (pass == 1 ? &map_b1 : (pass == 2 ? &map_b2 : &map_b3));
-          if (++kp == kb_per_pass) {
+          int bx = kk, by = n0;  // the W tile; on the diagonal its masked copy
+          if (tri && kp >= 2 * tn) {
+            mb = &map_d;
+            bx = kk - 2 * tn * BK_BYTES;
+            by = pass * drows + n0;
+          }
+          if (++kp == kbt) {
             kp = 0;
             ++pass;
           }
@@ -232,14 +263,14 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
             if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * SB);
             const uint32_t bar = smem_u32(&full_bar[s]) & kPeerMask;
             tma_load_2d_pair(dst, &map_a, bar, kk, m0);
-            tma_load_2d_pair(dst + A_STAGE, mb, bar, kk, n0);
+            tma_load_2d_pair(dst + A_STAGE, mb, bar, bx, by);
           } else if constexpr (FUSED) {
             mbar_expect_tx(&full_bar[s], B_STAGE);  // the producers write the A tile
-            tma_load_2d(dst + A_STAGE, mb, &full_bar[s], kk, n0);
+            tma_load_2d(dst + A_STAGE, mb, &full_bar[s], bx, by);
           } else {
             mbar_expect_tx(&full_bar[s], STAGE_BYTES);
             tma_load_2d(dst, &map_a, &full_bar[s], kk, m0);
-            tma_load_2d(dst + A_STAGE, mb, &full_bar[s], kk, n0);
+            tma_load_2d(dst + A_STAGE, mb, &full_bar[s], bx, by);
           }
         }
       }
@@ -254,6 +285,7 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
       bool ok = true;
       const int units_total = (t_end - t_begin) * upt;
       for (int u = 0; u < units_total && ok; ++u, ++i) {
+        const int spu = ppu * tile_kb((t_begin + u / upt) % ntn);  // stages of this accumulation
         const int a = i & 1;
         if (i >= 2 && !mbar_wait(&acce_bar[a], ((i >> 1) - 1) & 1)) {
           ok = false;
@@ -306,6 +338,7 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
     // the bits is hidden behind PF stages of MMAs.
     const int p = threadIdx.x - 192;
     constexpr int WPS = kInt8 ? 4 : 2;  // packed words per stage
+    const int kblocks = upt * ppu * kb_per_pass;  // (this form never runs triangular)
     const int nstage = (t_end - t_begin) * kblocks;
     // ring slot layout [slot][word q][thread p]: a warp's copies of one word
     // fall on 32 consecutive banks
@@ -388,6 +421,7 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
     cp_async_wait<0>();
   } else {
     // ---- epilogue: warps 2-5, all 128 threads take every branch together ----
+    pdl_wait();  // the zeroed control words
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     // q of this thread's candidate over the CTA's tiles of the current block
@@ -583,7 +617,10 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
                    "r"(ACC_COLS));
     }
   }
-  if (threadIdx.x == 0 && s_fail) atomicExch(err, 1);
+  if (threadIdx.x == 0 && s_fail) {
+    pdl_wait();
+    atomicExch(err, 1);
+  }
 }
 
 // One packed word -> 32 +-1 elements of the A operand.
@@ -613,18 +650,42 @@ __device__ __forceinline__ void expand_word(uint32_t bits, T* __restrict__ dst) 
   }
 }
 
-// Packed candidates -> the +-1 A operand (int8, or bf16 for the float path),
-// row pitch ld elements: one word per thread, so a warp's stores cover
-// contiguous 32-byte (int8) or 64-byte (bf16) pieces of a row. Columns at and
-// beyond n are never read (the A tensor map ends at n).
+// Before the GEMM, in one launch: the packed candidates -> the +-1 A operand
+// (int8, or bf16 for the float path), row pitch ld elements: one word per
+// thread, so a warp's stores cover contiguous 32-byte (int8) or 64-byte (bf16)
+// pieces of a row (columns at and beyond n are never read: the A tensor map
+// ends at n); the zeroed control words; and for the triangular form (D) the
+// strictly upper part of every plane's diagonal tiles: row j of a plane (`drows`
+// rows, zero from n on), column c: W[j][i], i = BN (j / BN) + c, where i < j,
+// else 0. The GEMM is a programmatic dependent: its set-up overlaps this kernel.
 template <typename T>
-__global__ void expand_pm1_kernel(const uint32_t* __restrict__ theta, int shots, int n32, int ld,
-                                  T* __restrict__ X) {
+__global__ void expand_pm1_kernel(const uint32_t* __restrict__ theta, int shots, int n32, int ld, T* __restrict__ X,
+                                  unsigned* __restrict__ ctl, int ctl_words, const int8_t* __restrict__ W, int n,
+                                  int planes, int drows, int8_t* __restrict__ D) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   const long long total = (long long)shots * n32;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
+  for (long long e = first; e < total; e += step) {
     const int b = (int)(e / n32), w = (int)(e - (long long)b * n32);
     expand_word<T>(__ldg(theta + e), X + (size_t)b * ld + (size_t)w * 32);
+  }
+  for (long long e = first; e < ctl_words; e += step) ctl[e] = 0u;
+  if (D) {
+    const int chunks = planes * drows * (BN / 16);  // 16 columns each
+    for (long long e = first; e < chunks; e += step) {
+      const int row = (int)(e / (BN / 16)), c0 = (int)(e % (BN / 16)) * 16;
+      const int pl = row / drows, j = row - pl * drows, i0 = j / BN * BN + c0;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (j < n && i0 < j) {  // (i0 < j < n: inside the padded row, 16-byte aligned)
+        v = __ldg(reinterpret_cast<const uint4*>(W + ((size_t)pl * n + j) * ld + i0));
+        const int keep = j - i0;  // bytes below the diagonal
+        uint32_t* p = &v.x;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          p[q] &= keep >= 4 * q + 4 ? 0xFFFFFFFFu : keep <= 4 * q ? 0u : (1u << (8 * (keep - 4 * q))) - 1u;
+      }
+      *reinterpret_cast<uint4*>(D + (size_t)row * BN + c0) = v;
+    }
   }
 }
 
@@ -672,11 +733,12 @@ struct MapCacheEntry {
   CUtensorMap map;
 };
 
-// Tensor maps depend only on (address, shape): keep the last few encoded.
+// Tensor maps depend only on (address, shape): each thread keeps the last few
+// encoded.
 bool cached_map(CUtensorMap* out, const void* base, bool int8, int rows, int cols, int pitch,
                 int box_rows) {
-  static MapCacheEntry cache[8] = {};
-  static int next = 0;
+  static thread_local MapCacheEntry cache[32] = {};
+  static thread_local int next = 0;
   for (const auto& e : cache) {
     if (e.base == base && e.rows == rows && e.cols == cols && e.pitch == pitch &&
         e.box_rows == box_rows && e.int8 == int8) {
@@ -687,7 +749,7 @@ bool cached_map(CUtensorMap* out, const void* base, bool int8, int rows, int col
   MapCacheEntry e{base, rows, cols, pitch, box_rows, int8, {}};
   if (!make_map(&e.map, base, int8, rows, cols, pitch, box_rows)) return false;
   cache[next] = e;
-  next = (next + 1) % 8;
+  next = (next + 1) % 32;
   *out = e.map;
   return true;
 }
@@ -719,7 +781,6 @@ pqi_status score_tc(const pqi_weights* w, const uint32_t* theta, int shots, int 
   const bool digits = w->kind != PQI_W_I8 && w->W_d && g_score_path != 4;
   const bool i8 = w->kind == PQI_W_I8 || digits;
   const int planes = digits ? 4 : 1;
-  const double qscale = digits ? w->wscale : 1.0;
   // the int8 epilogue sums 256 columns of |Y| <= 127 n in 32 bits
   if (i8 && n > 65536) return PQI_ENOTSUP;
   const int ntn = (n + tc::BN - 1) / tc::BN;
@@ -738,6 +799,14 @@ pqi_status score_tc(const pqi_weights* w, const uint32_t* theta, int shots, int 
   if (!fused)
     X = i8 ? (void*)ws.take<int8_t>((size_t)shots * ld) : (void*)ws.take<uint16_t>((size_t)shots * ld);
   if (!ctl || !qpart || (!fused && !X)) return PQI_EINVAL;
+  // Triangular form (int8 operands): W is symmetric, so q = 2 sum_j x_j
+  // sum_{i < j} W_ij x_i, and node tile t needs K only up to its own end, with
+  // its diagonal tile masked to i < j: (T + 1) / 2T of the MMAs for T node tiles
+  // (0.56 at n = 2048, 0.52 at 8192). Taken wherever there are two tiles or more
+  // and the workspace holds the masked tiles.
+  const int drows = ntn * tc::BN;
+  int8_t* D = i8 && !fused && ntn > 1 ? ws.take<int8_t>((size_t)planes * drows * tc::BN) : nullptr;
+  const int tri = D ? 1 : 0;
   int* err = reinterpret_cast<int*>(ctl);
   unsigned* mdone = reinterpret_cast<unsigned*>(ctl + 8);
   unsigned long long* key = reinterpret_cast<unsigned long long*>(ctl + 16);
@@ -755,11 +824,17 @@ pqi_status score_tc(const pqi_weights* w, const uint32_t* theta, int shots, int 
   const void* b1 = digits ? (const void*)(w->W_d + plane_bytes) : (i8 ? b0 : (const void*)w->W_lo);
   const void* b2 = digits ? (const void*)(w->W_d + 2 * plane_bytes) : b1;
   const void* b3 = digits ? (const void*)(w->W_d + 3 * plane_bytes) : b2;
-  CUtensorMap ma, mb0, mb1, mb2, mb3;
+  const double qscale = (digits ? w->wscale : 1.0) * (tri ? 2.0 : 1.0);
+  CUtensorMap ma, mb0, mb1, mb2, mb3, md;
   if (!cached_map(&mb0, b0, i8, n, n, ld, brows)) return PQI_ENOTSUP;
   if (!cached_map(&mb1, b1, i8, n, n, ld, brows)) return PQI_ENOTSUP;
   if (!cached_map(&mb2, b2, i8, n, n, ld, brows)) return PQI_ENOTSUP;
   if (!cached_map(&mb3, b3, i8, n, n, ld, brows)) return PQI_ENOTSUP;
+  if (!tri) {
+    md = mb0;  // not read
+  } else if (!cached_map(&md, D, true, planes * drows, tc::BN, tc::BN, brows)) {
+    return PQI_ENOTSUP;
+  }
   if (fused) {
     ma = mb0;  // not read: the kernel writes its A tiles itself
   } else if (!cached_map(&ma, X, i8, shots, n, ld, tc::BM)) {
@@ -778,31 +853,35 @@ pqi_status score_tc(const pqi_weights* w, const uint32_t* theta, int shots, int 
     PQI_TRY(cudaFuncSetAttribute(kfn[i8][form], cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
     attr_set[i8][form] = true;
   }
-  PQI_TRY(cudaMemsetAsync(ctl, 0, ctl_bytes, s));
-  if (!fused) {
-    const long long words = (long long)shots * n32;
+  if (fused) {
+    PQI_TRY(cudaMemsetAsync(ctl, 0, ctl_bytes, s));
+  } else {
+    const long long words = (long long)shots * n32 + (long long)planes * tri * drows * (tc::BN / 16);
     const int eg = (int)std::max<long long>(1, std::min<long long>((words + 255) / 256, 148 * 16));
+    const int8_t* wd = static_cast<const int8_t*>(b0);
+    unsigned* cw = reinterpret_cast<unsigned*>(ctl);
+    const int cn = (int)(ctl_bytes / sizeof(unsigned));
     if (i8) {
-      tc::expand_pm1_kernel<int8_t><<<eg, 256, 0, s>>>(theta, shots, n32, ld, (int8_t*)X);
+      tc::expand_pm1_kernel<int8_t><<<eg, 256, 0, s>>>(theta, shots, n32, ld, (int8_t*)X, cw, cn, wd, n, planes, drows, D);
     } else {
-      tc::expand_pm1_kernel<uint16_t><<<eg, 256, 0, s>>>(theta, shots, n32, ld, (uint16_t*)X);
+      tc::expand_pm1_kernel<uint16_t><<<eg, 256, 0, s>>>(theta, shots, n32, ld, (uint16_t*)X, cw, cn, nullptr, n, 0, 0, nullptr);
     }
     PQI_LAUNCHED("expand_pm1_kernel");
   }
   const int limit = g_score_grid > 0 ? g_score_grid : num_sms;
   if (g_score_ev_before) PQI_TRY(cudaEventRecord(g_score_ev_before, s));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  cfg.stream = s;
+  cfg.blockDim = dim3(fused ? tc::FTHREADS : tc::PTHREADS);
+  cfg.dynamicSmemBytes = smem_bytes;
   if (pair) {
     const int tiles = ntn * ((shots + 2 * tc::BM - 1) / (2 * tc::BM));
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(tc::PTHREADS);
-    cfg.dynamicSmemBytes = tc::SMEM_BYTES;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
     cfg.numAttrs = 1;
     // a persistent grid of exactly the pairs that can be resident at once (a
     // pair needs two free SMs of one GPC), cached per weight kind
@@ -813,31 +892,29 @@ pqi_status score_tc(const pqi_weights* w, const uint32_t* theta, int shots, int 
       PQI_TRY(cudaOccupancyMaxActiveClusters(&f, kfn[i8][2], &cfg));
       fit[i8] = std::max(1, f);
     }
-    const int pairs = std::max(1, std::min({tiles, limit / 2, fit[i8]}));
-    cfg.gridDim = dim3(2 * pairs);
-    if (i8) {
-      PQI_TRY(cudaLaunchKernelEx(&cfg, tc::score_tc_kernel<true, true, false>, ma, mb0, mb1, mb2, mb3, planes, qscale, n, shots,
-                                 theta, n32, w->upper_sum, spin, geo, qpart, energies, mcount,
-                                 mdone, key, best_energy, best_index, err));
-    } else {
-      PQI_TRY(cudaLaunchKernelEx(&cfg, tc::score_tc_kernel<false, true, false>, ma, mb0, mb1, mb2, mb3, planes, qscale, n, shots,
-                                 theta, n32, w->upper_sum, spin, geo, qpart, energies, mcount,
-                                 mdone, key, best_energy, best_index, err));
-    }
+    cfg.gridDim = dim3(2 * std::max(1, std::min({tiles, limit / 2, fit[i8]})));
   } else {
-    const int grid = std::min(ntn * ntm, limit);
-    const int threads = fused ? tc::FTHREADS : tc::PTHREADS;
-    if (i8) {
-      auto k = fused ? tc::score_tc_kernel<true, false, true> : tc::score_tc_kernel<true, false, false>;
-      k<<<grid, threads, smem_bytes, s>>>(ma, mb0, mb1, mb2, mb3, planes, qscale, n, shots, theta, n32, w->upper_sum, spin, geo,
-                                          qpart, energies, mcount, mdone, key, best_energy, best_index,
-                                          err);
-    } else {
-      auto k = fused ? tc::score_tc_kernel<false, false, true> : tc::score_tc_kernel<false, false, false>;
-      k<<<grid, threads, smem_bytes, s>>>(ma, mb0, mb1, mb2, mb3, planes, qscale, n, shots, theta, n32, w->upper_sum, spin, geo,
-                                          qpart, energies, mcount, mdone, key, best_energy, best_index,
-                                          err);
-    }
+    cfg.gridDim = dim3(std::min(ntn * ntm, limit));
+  }
+  // behind the expansion pass (and no event between the two)
+  if (!fused && !g_score_ev_before) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  auto launch = [&](auto k) {
+    return cudaLaunchKernelEx(&cfg, k, ma, mb0, mb1, mb2, mb3, md, tri, planes, qscale, n, shots, theta, n32,
+                              w->upper_sum, spin, geo, qpart, energies, mcount, mdone, key, best_energy, best_index,
+                              err);
+  };
+  if (i8) {
+    PQI_TRY(pair ? launch(tc::score_tc_kernel<true, true, false>)
+            : fused ? launch(tc::score_tc_kernel<true, false, true>)
+                    : launch(tc::score_tc_kernel<true, false, false>));
+  } else {
+    PQI_TRY(pair ? launch(tc::score_tc_kernel<false, true, false>)
+            : fused ? launch(tc::score_tc_kernel<false, false, true>)
+                    : launch(tc::score_tc_kernel<false, false, false>));
   }
   PQI_LAUNCHED("score_tc_kernel");
   if (g_score_ev_after) PQI_TRY(cudaEventRecord(g_score_ev_after, s));
