@@ -87,6 +87,138 @@ __global__ void __launch_bounds__(256) gemm_bf16_kernel(int transA, int transB, 
   }
 }
 
+// The same product for the shapes of one graph, where 64 x 64 tiles leave most
+// of the chip idle (the weight gradients, K = n, are one or two tiles): a warp
+// per 16 x 8 tile, four outputs per lane, the next chunk of 128 k loaded to
+// registers in 16-byte vectors while the current one is multiplied. (Larger
+// tiles were bound by shared memory: four warps reading the same operands.)
+// Every output is the same chain of float32 fused multiply-adds over ascending
+// k as above, so the values are the same bits; that chain bounds it.
+constexpr int SM_TM = 16, SM_TN = 8, SM_TK = 128, SM_THREADS = 32;
+constexpr int SM_MAX_TILES = 296;  // 64 x 64 tiles: two per SM
+
+// Eight consecutive bf16 of a row, those from `valid` on zero: one 16-byte load
+// where the row is aligned (vec) and holds them all.
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, int valid, bool vec) {
+  if (vec && valid >= 8) return __ldg(reinterpret_cast<const uint4*>(p));
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (i < valid) w[i >> 1] |= (uint32_t)__bfloat16_as_ushort(p[i]) << (16 * (i & 1));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__device__ __forceinline__ void to_float8(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {  // (a bf16 is the high half of its float)
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+
+// vecA / vecB: 16-byte aligned base and row pitch.
+template <bool transA, bool transB>
+__global__ void __launch_bounds__(SM_THREADS) gemm_bf16_small_kernel(
+    int M, int N, int K, float alpha, const __nv_bfloat16* __restrict__ A, int lda, bool vecA,
+    const __nv_bfloat16* __restrict__ B, int ldb, bool vecB, float beta, float* C32, __nv_bfloat16* C16, int ldc,
+    const float* __restrict__ bias, int relu) {
+  constexpr int AV = SM_TK * SM_TM / 8 / SM_THREADS, BV = SM_TK * SM_TN / 8 / SM_THREADS;  // vectors per thread
+  __shared__ __align__(16) float As[SM_TK][SM_TM + 4];
+  __shared__ __align__(16) float Bs[SM_TK][SM_TN + 4];
+  const int mg = threadIdx.x & 3, nn = threadIdx.x >> 2;  // outputs m0 + 4 mg .. + 3, n0 + nn
+  const int m0 = blockIdx.y * SM_TM, n0 = blockIdx.x * SM_TN;
+  uint4 ra[AV], rb[BV];
+  // Vector e of a tile runs along the operand's contiguous dimension: along m
+  // (n) for a transposed A (a plain B), else along k with neighbouring threads
+  // on neighbouring rows, so that their stores fall on different banks.
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int i = 0; i < AV; ++i) {
+      const int e = threadIdx.x + i * SM_THREADS;
+      if constexpr (transA) {
+        const int k = k0 + e / (SM_TM / 8), m = m0 + e % (SM_TM / 8) * 8;
+        ra[i] = load8(A + (size_t)k * lda + m, k < K ? M - m : 0, vecA);
+      } else {
+        const int m = m0 + e % SM_TM, k = k0 + e / SM_TM * 8;
+        ra[i] = load8(A + (size_t)m * lda + k, m < M ? K - k : 0, vecA);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < BV; ++i) {
+      const int e = threadIdx.x + i * SM_THREADS;
+      if constexpr (!transB) {
+        const int k = k0 + e / (SM_TN / 8), n = n0 + e % (SM_TN / 8) * 8;
+        rb[i] = load8(B + (size_t)k * ldb + n, k < K ? N - n : 0, vecB);
+      } else {
+        const int n = n0 + e % SM_TN, k = k0 + e / SM_TN * 8;
+        rb[i] = load8(B + (size_t)n * ldb + k, n < N ? K - k : 0, vecB);
+      }
+    }
+  };
+  auto store = [&]() {
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < AV; ++i) {
+      const int e = threadIdx.x + i * SM_THREADS;
+      to_float8(ra[i], f);
+      if constexpr (transA) {
+        float4* d = reinterpret_cast<float4*>(&As[e / (SM_TM / 8)][e % (SM_TM / 8) * 8]);
+        d[0] = make_float4(f[0], f[1], f[2], f[3]);
+        d[1] = make_float4(f[4], f[5], f[6], f[7]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) As[e / SM_TM * 8 + j][e % SM_TM] = f[j];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < BV; ++i) {
+      const int e = threadIdx.x + i * SM_THREADS;
+      to_float8(rb[i], f);
+      if constexpr (!transB) {
+        float4* d = reinterpret_cast<float4*>(&Bs[e / (SM_TN / 8)][e % (SM_TN / 8) * 8]);
+        d[0] = make_float4(f[0], f[1], f[2], f[3]);
+        d[1] = make_float4(f[4], f[5], f[6], f[7]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) Bs[e / SM_TN * 8 + j][e % SM_TN] = f[j];
+      }
+    }
+  };
+  float acc[4] = {};
+  load(0);
+  for (int k0 = 0; k0 < K; k0 += SM_TK) {
+    store();
+    __syncwarp();
+    if (k0 + SM_TK < K) load(k0 + SM_TK);
+    // (k past K: zero operands leave the sums as they are, as above)
+    const int kn = min(SM_TK, (K - k0 + 15) & ~15);
+#pragma unroll 16
+    for (int kk = 0; kk < kn; ++kk) {
+      const float4 a = *reinterpret_cast<const float4*>(&As[kk][4 * mg]);
+      const float b = Bs[kk][nn];
+      acc[0] = fmaf(a.x, b, acc[0]);
+      acc[1] = fmaf(a.y, b, acc[1]);
+      acc[2] = fmaf(a.z, b, acc[2]);
+      acc[3] = fmaf(a.w, b, acc[3]);
+    }
+    __syncwarp();
+  }
+  const int n = n0 + nn;
+  if (n >= N) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + 4 * mg + i;
+    if (m >= M) continue;
+    float v = alpha * acc[i];
+    if (beta != 0.0f) v += beta * C32[(size_t)m * ldc + n];
+    if (bias) v += bias[n];
+    if (relu) v = fmaxf(v, 0.0f);
+    if (C32) C32[(size_t)m * ldc + n] = v;
+    if (C16) C16[(size_t)m * ldc + n] = __float2bfloat16_rn(v);
+  }
+}
+
 // row sums of |W| (caller's matrix, pitch n, diagonal ignored)
 __global__ void abs_rowsum_kernel(const float* __restrict__ W, int n, float* __restrict__ s) {
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -394,6 +526,27 @@ pqi_status pqi_mpnn_gemm(int transA, int transB, int M, int N, int K, float alph
   PQI_CHECK_ARG(A && B && (C32 || C16) && M > 0 && N > 0 && K > 0);
   PQI_CHECK_ARG(beta == 0.0f || C32);
   dim3 grid((N + mp::TN - 1) / mp::TN, (M + mp::TM - 1) / mp::TM);
+  // Below two 64 x 64 tiles per SM the warp tiles are faster at every shape of
+  // the network (n 128 to 16384). Per gradient (K = n = 1024, 128 x 64 outputs)
+  // 120 us -> 16 us; a training example (forward and backward) n = 1024 887 ->
+  // 400 us, of which 330 is the host's launches, n = 4096 2818 -> 809, n = 16384
+  // 13.0 -> 3.1 ms.
+  if ((long long)grid.x * grid.y < mp::SM_MAX_TILES) {
+    const dim3 small((N + mp::SM_TN - 1) / mp::SM_TN, (M + mp::SM_TM - 1) / mp::SM_TM);
+    auto aligned = [](const void* p, int ld) { return ((uintptr_t)p & 15) == 0 && ld % 8 == 0; };
+    auto launch = [&](auto kern) {
+      kern<<<small, mp::SM_THREADS, 0, as_stream(stream)>>>(
+          M, N, K, alpha, static_cast<const __nv_bfloat16*>(A), lda, aligned(A, lda),
+          static_cast<const __nv_bfloat16*>(B), ldb, aligned(B, ldb), beta, C32, static_cast<__nv_bfloat16*>(C16), ldc, bias, relu);
+    };
+    if (transA) {
+      transB ? launch(mp::gemm_bf16_small_kernel<true, true>) : launch(mp::gemm_bf16_small_kernel<true, false>);
+    } else {
+      transB ? launch(mp::gemm_bf16_small_kernel<false, true>) : launch(mp::gemm_bf16_small_kernel<false, false>);
+    }
+    PQI_LAUNCHED("gemm_bf16_small_kernel");
+    return PQI_OK;
+  }
   mp::gemm_bf16_kernel<<<grid, 256, 0, as_stream(stream)>>>(
       transA, transB, M, N, K, alpha, static_cast<const __nv_bfloat16*>(A), lda,
       static_cast<const __nv_bfloat16*>(B), ldb, beta, C32, static_cast<__nv_bfloat16*>(C16), ldc,
