@@ -302,96 +302,114 @@ __device__ __forceinline__ void flip_and_select(const TaskCtx<WT, GT>& c, int k,
 // Y[t][v] = sum_u x_tu W[u][v] (x = +-1), u ascending from 0 - the order and
 // the accumulation type (float64 for float weights, int32 for int8) of the
 // search kernel's own column-order sum, so the fields are the same numbers.
-// A CTA takes SF_T tasks x SF_V nodes: each row chunk of W (SF_U rows) is
-// read once into shared memory (converted once) and used by all SF_T tasks,
-// instead of every task streaming all of W. The tasks of a tile may belong to
-// different graphs: the tile runs once per distinct graph among its tasks
-// (one pass for tasks grouped by graph). Row-list graphs are skipped (the
-// search kernel sums their nonzeros itself).
-constexpr int SF_T = 64;
-constexpr int SF_V = 64;
+// Bound by the float64 pipe (64 lanes per clock per SM). A CTA takes ST tasks x
+// 16 VI nodes: each chunk of SF_U rows of W is read once into shared memory
+// (converted once, the next chunk's loads in flight meanwhile) and used by all
+// ST tasks. A thread holds TJ tasks x VI nodes, nodes 16 apart so that a warp's
+// reads of a row are contiguous; with 8 x 4 the 32 multiply-adds per 4 reads
+// keep shared memory at half the float64 pipe's time (4 x 4 with four
+// neighbouring nodes per thread read it conflicted, at twice that time, and
+// waited for every chunk). Float32 n = 8192: 32 tasks 1606 -> 322 us, 8 tasks
+// 1597 -> 222, 592 tasks 5.8 -> 4.0 ms; n = 5999, 592 tasks 3.8 -> 2.3 ms (0.56 of
+// the float64 rate). The tasks of a
+// tile may belong to different graphs: the tile runs once per distinct graph
+// among its tasks (one pass for tasks grouped by graph). Row-list graphs are
+// skipped (the search kernel sums their nonzeros itself).
 constexpr int SF_U = 32;
+constexpr int sf_threads(int ST, int TJ) { return 16 * (ST / TJ); }  // 16 node columns x task rows
 
-template <typename WT>
-__global__ void __launch_bounds__(256) start_fields_kernel(
+template <typename WT, int ST, int TJ, int VI>
+__global__ void __launch_bounds__(sf_threads(ST, TJ)) start_fields_kernel(
     const BatchGraph* __restrict__ graphs, const int* __restrict__ task_graph,
     const uint32_t* __restrict__ init_states, int words_pitch, int tasks,
     double* __restrict__ Y, int ypitch) {
   typedef typename std::conditional<sizeof(WT) == 1, int, double>::type AT;
-  __shared__ __align__(16) AT Ws[SF_U][SF_V];
-  __shared__ uint32_t Xs[SF_T];
-  __shared__ int gid[SF_T];
-  const int t0 = blockIdx.x * SF_T, v0 = blockIdx.y * SF_V;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // nodes v0+4tx+i, tasks t0+4ty+j
-  if (threadIdx.x < SF_T) gid[threadIdx.x] = t0 + (int)threadIdx.x < tasks ? task_graph[t0 + threadIdx.x] : -1;
+  typedef typename std::conditional<sizeof(WT) == 1, char4, float4>::type V4;
+  constexpr int SF_V = 16 * VI, NT = sf_threads(ST, TJ), VPT = SF_U * SF_V / 4 / NT;  // vectors of a chunk per thread
+  __shared__ __align__(16) AT Ws[2][SF_U][SF_V];
+  __shared__ int gid[ST];
+  const int t0 = blockIdx.x * ST, v0 = blockIdx.y * SF_V;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // nodes v0 + tx + 16 i, tasks t0 + TJ ty + j
+  for (int i = threadIdx.x; i < ST; i += NT) gid[i] = t0 + i < tasks ? task_graph[t0 + i] : -1;
   __syncthreads();
+  constexpr uint64_t kAll = ST == 64 ? ~0ull : (1ull << (ST & 63)) - 1ull;
   uint64_t done = 0;  // tile tasks handled (the same in every thread)
-  for (int i = 0; i < SF_T; ++i)
+  for (int i = 0; i < ST; ++i)
     if (gid[i] < 0) done |= 1ull << i;
-  while (done != ~0ull) {
+  while (done != kAll) {
     const int g = gid[__ffsll((long long)~done) - 1];
     uint64_t mine = 0;
-    for (int i = 0; i < SF_T; ++i)
+    for (int i = 0; i < ST; ++i)
       if (gid[i] == g) mine |= 1ull << i;
     done |= mine;
     const BatchGraph G = graphs[g];
     if (G.adj_ptr || v0 >= G.n) continue;
     const WT* __restrict__ W = static_cast<const WT*>(G.W);
     const int n = G.n;
-    AT acc[4][4];
+    const uint32_t mj = (uint32_t)(mine >> (TJ * ty)) & ((1u << TJ) - 1u);
+    AT acc[VI][TJ];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < VI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0;
-    for (int u0 = 0; u0 < n; u0 += SF_U) {
-      __syncthreads();  // the previous chunk's reads are done
-      for (int idx = threadIdx.x; idx < SF_U * SF_V; idx += blockDim.x) {
-        const int r = idx / SF_V, c = idx - r * SF_V;
-        const int u = u0 + r, v = v0 + c;
-        Ws[r][c] = (u < n && v < n) ? (AT)__ldg(W + (size_t)u * G.ld + v) : (AT)0;
+      for (int j = 0; j < TJ; ++j) acc[i][j] = 0;
+    V4 wr[VPT];
+    uint32_t xn[TJ];
+    auto load = [&](int u0) {  // (rows are zero padded to a multiple of 128 columns)
+#pragma unroll
+      for (int q = 0; q < VPT; ++q) {
+        const int e = threadIdx.x + q * NT, r = e / (SF_V / 4), c = e % (SF_V / 4) * 4;
+        wr[q] = V4{0, 0, 0, 0};
+        if (u0 + r < n) wr[q] = __ldg(reinterpret_cast<const V4*>(W + (size_t)(u0 + r) * G.ld + v0 + c));
       }
-      if (threadIdx.x < SF_T)
-        Xs[threadIdx.x] = ((mine >> threadIdx.x) & 1ull)
-                              ? __ldg(init_states + (size_t)(t0 + threadIdx.x) * words_pitch + (u0 >> 5))
-                              : 0u;
-      __syncthreads();
-      uint32_t xw[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) xw[j] = Xs[4 * ty + j];
+      for (int j = 0; j < TJ; ++j)
+        xn[j] = ((mj >> j) & 1u) ? __ldg(init_states + (size_t)(t0 + TJ * ty + j) * words_pitch + (u0 >> 5)) : 0u;
+    };
+    __syncthreads();  // the reads of the graph before are done
+    load(0);
+    for (int u0 = 0; u0 < n; u0 += SF_U) {
+      AT(*Wc)[SF_V] = Ws[(u0 / SF_U) & 1];
+#pragma unroll
+      for (int q = 0; q < VPT; ++q) {
+        const int e = threadIdx.x + q * NT, r = e / (SF_V / 4), c = e % (SF_V / 4) * 4;
+        Wc[r][c] = (AT)wr[q].x;
+        Wc[r][c + 1] = (AT)wr[q].y;
+        Wc[r][c + 2] = (AT)wr[q].z;
+        Wc[r][c + 3] = (AT)wr[q].w;
+      }
+      uint32_t xw[TJ];
+#pragma unroll
+      for (int j = 0; j < TJ; ++j) xw[j] = xn[j];
+      __syncthreads();  // (the other buffer's readers passed the barrier before)
+      if (u0 + SF_U < n) load(u0 + SF_U);
       // acc += (+-1) w as one fused multiply-add with an exact product: the
-      // same rounding as the add of +-w, and the sign is chosen once per task
-      // and row instead of once per element
-      auto row = [&](int r) {
-        AT w[4];
+      // same rounding as the add of +-w; rows past n are zero and change nothing
+#pragma unroll 16
+      for (int r = 0; r < SF_U; ++r) {
+        AT w[VI];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = Ws[r][4 * tx + i];
+        for (int i = 0; i < VI; ++i) w[i] = Wc[r][tx + 16 * i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const AT sj = ((xw[j] >> r) & 1u) ? (AT)1 : (AT)-1;
+        for (int j = 0; j < TJ; ++j) {
+          if constexpr (std::is_same<AT, double>::value) {
+            const double sj = __hiloint2double(((xw[j] >> r) & 1u) ? 0x3FF00000 : (int)0xBFF00000, 0);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if constexpr (std::is_same<AT, double>::value) {
-              acc[i][j] = fma(sj, w[i], acc[i][j]);
-            } else {
-              acc[i][j] += sj * w[i];
-            }
+            for (int i = 0; i < VI; ++i) acc[i][j] = fma(sj, w[i], acc[i][j]);
+          } else {
+            const int sj = ((xw[j] >> r) & 1u) ? 1 : -1;
+#pragma unroll
+            for (int i = 0; i < VI; ++i) acc[i][j] += sj * w[i];
           }
         }
-      };
-      if (n - u0 >= SF_U) {
-#pragma unroll 8
-        for (int r = 0; r < SF_U; ++r) row(r);
-      } else {
-        for (int r = 0; r < n - u0; ++r) row(r);
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (!((mine >> (4 * ty + j)) & 1ull)) continue;
-      const int t = t0 + 4 * ty + j;
+    for (int j = 0; j < TJ; ++j) {
+      if (!((mj >> j) & 1u)) continue;
+      const int t = t0 + TJ * ty + j;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int v = v0 + 4 * tx + i;
+      for (int i = 0; i < VI; ++i) {
+        const int v = v0 + tx + 16 * i;
         if (v < n) Y[(size_t)t * ypitch + v] = (double)acc[i][j];
       }
     }
@@ -1192,11 +1210,18 @@ pqi_status pqi::start_fields(const void* graphs, const int* task_graph,
   const int yp = (max_n + 3) & ~3;
   double* y = nullptr;
   PQI_TRY(cudaMallocAsync(reinterpret_cast<void**>(&y), (size_t)tasks * yp * sizeof(double), s));
-  const dim3 grid((unsigned)((tasks + SF_T - 1) / SF_T), (unsigned)((max_n + SF_V - 1) / SF_V));
-  if (i8) {
-    start_fields_kernel<int8_t><<<grid, 256, 0, s>>>(gd, task_graph, init_states, words_pitch, tasks, y, yp);
+  auto launch = [&](auto kern, int ST, int TJ, int VI) {
+    const dim3 grid((unsigned)((tasks + ST - 1) / ST), (unsigned)((max_n + 16 * VI - 1) / (16 * VI)));
+    kern<<<grid, sf_threads(ST, TJ), 0, s>>>(gd, task_graph, init_states, words_pitch, tasks, y, yp);
+  };
+  // Few tasks: tiles that hold just them, with fewer sums per thread, so that
+  // the nodes still fill the chip.
+  if (tasks <= 16) {
+    i8 ? launch(start_fields_kernel<int8_t, 16, 2, 2>, 16, 2, 2) : launch(start_fields_kernel<float, 16, 2, 2>, 16, 2, 2);
+  } else if (tasks <= 32) {
+    i8 ? launch(start_fields_kernel<int8_t, 32, 4, 2>, 32, 4, 2) : launch(start_fields_kernel<float, 32, 4, 2>, 32, 4, 2);
   } else {
-    start_fields_kernel<float><<<grid, 256, 0, s>>>(gd, task_graph, init_states, words_pitch, tasks, y, yp);
+    i8 ? launch(start_fields_kernel<int8_t, 64, 8, 4>, 64, 8, 4) : launch(start_fields_kernel<float, 64, 8, 4>, 64, 8, 4);
   }
   PQI_LAUNCHED("start_fields_kernel");
   *out = y;
