@@ -12,25 +12,26 @@
 //      (y_v += coef * W_kv, one float4 / char4 of row k per group; the owner of
 //      k toggles its bit) and folds the new gains g_v = x_v y_v into a local
 //      argmax: float gain first, then the lowest node (a 64-bit key);
-//   2. warp maxima (two 32-bit redux steps) meet in shared memory behind one
-//      CTA barrier; warp 0 reduces them and lanes 0..C-1 write the CTA's best
-//      (key, exact gain) into slot [rank] of every CTA with st.async, which
-//      counts the bytes on that CTA's mbarrier;
-//   3. thread 0 waits (bounded) for the C slots of the flip, a second CTA
-//      barrier (which also spreads a failed wait) releases the CTA, and every
-//      warp reduces the C local slots to the same global best, flipped next if
-//      its gain is > 0.
-// Two slot arrays and two mbarriers alternate between flips; a CTA can only be
-// one flip ahead of any other, so a slot array is never rewritten while read.
-// The selection rule is the batched kernel's (pqi_batch_search), so both give
-// the same trajectory. Control flow depends only on values every CTA reads
-// identically; the flip budget and the bounded waits end every loop.
+//   2. warp maxima (two 32-bit redux steps) meet in shared memory behind the
+//      flip's one CTA barrier; warp 0 reduces them and its lanes 0..C-1 write the
+//      CTA's best (key, exact gain) into slot [rank] of every CTA with st.async,
+//      which counts the bytes on that CTA's mbarrier;
+//   3. every warp waits (bounded) for the C slots of the flip and reduces them
+//      itself to the same global best, flipped next if its gain is > 0. (Warps
+//      that each sent to every CTA, with no barrier, took 1.2 times as long.)
+// Two slot arrays and two mbarriers alternate between flips; a CTA sends flip
+// f + 2 only after every CTA has sent f + 1, so all its warps have read f, and a
+// slot array is never rewritten while read. The selection rule is the batched
+// kernel's (pqi_batch_search), so both give the same trajectory. Control flow
+// depends only on values every warp reads identically; the flip budget and the
+// bounded waits end every loop.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <type_traits>
 
 #include "pqi_common.cuh"
+#include "pqi_tc.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -59,7 +60,7 @@ struct Slot {
 };
 
 constexpr int kMaxCluster = 16;
-constexpr long long kWaitCycles = 2000000000ll;  // ~1 s: a cluster peer that stops writing
+constexpr int kMaxWarps = 8;  // per CTA
 
 __device__ __forceinline__ unsigned long long flip_key(float gv, int u, int xu) {
   return ((unsigned long long)ord_f32(gv) << 32) |
@@ -83,10 +84,6 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long ke
   return ((unsigned long long)hi << 32) | lo;
 }
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
 template <typename WT, int NG>
 __global__ void __launch_bounds__(256) cluster_ascent_kernel(
     const ClusterGraph* __restrict__ graphs, const int* __restrict__ task_graph,
@@ -101,23 +98,22 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
   extern __shared__ __align__(16) unsigned char smem[];
   // slots[p][r]: CTA r's best of the flips with parity p, written here by CTA r
   __shared__ __align__(16) Slot slots[2][kMaxCluster];
-  __shared__ __align__(8) unsigned long long bar[2];
+  __shared__ unsigned long long red_key[kMaxWarps];
+  __shared__ __align__(8) uint64_t bar[2];
   __shared__ double qslot[kMaxCluster];
-  __shared__ unsigned long long red_key[8];
-  __shared__ double red_g[8];
+  __shared__ double red_g[kMaxWarps];
   __shared__ int abort_flag;
   __shared__ int stop_flag;  // written by rank 0 (target mode)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int T = blockDim.x, nwarps = T >> 5;
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar[0])));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar[1])));
+    tc::mbar_init(&bar[0], 1);
+    tc::mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_flag = 0;
   }
   cl.sync();
-  uint32_t phase = 0;  // bit p: parity of bar[p]'s current phase
-  int par = 0;
+  uint32_t seq = 0;  // exchanges so far (over all tasks)
   const int clusters = gridDim.x / C;
   for (int task = blockIdx.x / C; task < tasks; task += clusters) {
     const ClusterGraph G = graphs[task_graph[task]];
@@ -182,6 +178,7 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
     int timeout = 0, failed = 0;
     int k = -1;
     GT coef = 0;
+    double gk = 0.0;
     for (int f = 0;; ++f) {
       if (k >= 0) {
         // apply the previous flip (node k) to my fields
@@ -255,20 +252,17 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
       const unsigned long long wkey = warp_max_key(key);
       if (lane == 0) red_key[warp] = wkey;
       if (key != 0ull && key == wkey) red_g[warp] = bg;
-      // arm this flip's barrier: C slots of 16 bytes are expected
-      if (threadIdx.x == 0)
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                         smem_addr(&bar[par])),
-                     "r"(C * (int)sizeof(Slot))
-                     : "memory");
+      const uint32_t par = seq & 1u, ph = (seq >> 1) & 1u;
+      ++seq;
+      if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(C * sizeof(Slot)));
       __syncthreads();
-      int bad = 0;
       if (warp == 0) {
+        // this CTA's best into slot [rank] of every CTA, counted on its bar[par]
         const unsigned long long ck = lane < nwarps ? red_key[lane] : 0ull;
         const double cgv = lane < nwarps ? red_g[lane] : 0.0;
         const unsigned long long cb = warp_max_key(ck);
-        const uint32_t src = __ballot_sync(0xFFFFFFFFu, ck == cb && cb != 0ull);
-        const double cbg = __shfl_sync(0xFFFFFFFFu, cgv, src ? __ffs(src) - 1 : 0);
+        const uint32_t src = __ballot_sync(0xFFFFFFFFu, ck == cb);
+        const double cbg = __shfl_sync(0xFFFFFFFFu, cgv, __ffs(src) - 1);
         // the next row is one of the C CTAs' candidates: pull this CTA's
         // candidate row into L2 while the exchange is in flight (a hint only;
         // a row is ld * sizeof(WT) bytes, 16-byte aligned, inside W)
@@ -279,49 +273,29 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
                        : "memory");
         }
         if (lane < C) {
-          // this CTA's best into slot [rank] of CTA `lane`, counted on its bar[par]
           uint32_t raddr, rbar;
           asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
                        : "=r"(raddr)
-                       : "r"(smem_addr(&slots[par][rank])), "r"(lane));
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                       : "=r"(rbar)
-                       : "r"(smem_addr(&bar[par])), "r"(lane));
+                       : "r"(tc::smem_u32(&slots[par][rank])), "r"(lane));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[par])), "r"(lane));
           asm volatile(
-              "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, "
-              "[%3];" ::"r"(raddr),
+              "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
               "l"(cb), "l"(__double_as_longlong(cbg)), "r"(rbar)
               : "memory");
         }
-        if (lane == 0) {
-          // wait (bounded) for the C slots of this flip
-          const uint32_t ph = (phase >> par) & 1;
-          const long long t0 = clock64();
-          uint32_t done = 0;
-          while (true) {
-            asm volatile(
-                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                " selp.u32 %0, 1, 0, p;\n}"
-                : "=r"(done)
-                : "r"(smem_addr(&bar[par])), "r"(ph)
-                : "memory");
-            if (done || clock64() - t0 > kWaitCycles) break;
-          }
-          bad = !done;
-        }
       }
-      if (__syncthreads_or(bad)) {
-        failed = 1;
+      if (!tc::mbar_wait_spin(&bar[par], ph)) {
+        failed = 1;  // a peer stopped writing
         break;
       }
-      phase ^= 1u << par;
-      // the cluster's best (identical in every CTA)
+      // the cluster's best (identical in every warp)
       const unsigned long long sk = lane < C ? slots[par][lane].key : 0ull;
       const double sg = lane < C ? slots[par][lane].g : 0.0;
       const unsigned long long gkey = warp_max_key(sk);
-      const uint32_t gsrc = __ballot_sync(0xFFFFFFFFu, sk == gkey && gkey != 0ull);
-      const double gk = __shfl_sync(0xFFFFFFFFu, sg, gsrc ? __ffs(gsrc) - 1 : 0);
-      par ^= 1;
+      if (rank == 0 && warp == 0) {  // the value is kept by warp 0 of CTA 0
+        const uint32_t gsrc = __ballot_sync(0xFFFFFFFFu, sk == gkey);
+        gk = __shfl_sync(0xFFFFFFFFu, sg, __ffs(gsrc) - 1);
+      }
       if (gkey == 0ull || !(key_gain(gkey) > 0.0f)) break;
       if (f >= flip_budget) {
         timeout = 1;
@@ -344,7 +318,7 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
       wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 4);
       if ((lane & 7) == 0 && v0 < hi) bits[v0 >> 5] = wd;
     }
-    if (failed && threadIdx.x == 0) *cl.map_shared_rank(&abort_flag, 0) = 1;
+    if (failed && lane == 0) *cl.map_shared_rank(&abort_flag, 0) = 1;
     cl.sync();  // all slices final before rank 0 gathers the bits
     if (rank == 0) {
       for (int w = threadIdx.x; w < n32; w += T)
