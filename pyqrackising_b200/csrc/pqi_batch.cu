@@ -666,6 +666,12 @@ __global__ void __launch_bounds__(BT, (F32 ? 4 : 3) * 256 / BT) batch_search_ker
 // shared-memory form, so both return the same states, values and flip counts.
 // Each CTA asks for enough shared memory that no further CTA can join an SM
 // whose TMEM the resident CTAs hold.
+// What a flip takes: its row (0.7 us until the first chunk arrives), 19
+// instructions per node (a branch-free chunk of 16 nodes each; issue 0.6 of peak
+// with four tasks per SM) and the selection's barrier. With a branch per group
+// of four nodes and two conversions per node (16 lanes per clock per SM) the
+// passes took 2.5 times as long. SK 5999, 592 starts, 2 rounds of kicks: 16.6 ->
+// 12.2 ms; SK 8192, one start per SM: 5.1 -> 2.7 us per flip.
 // The shape per J (groups of four nodes per thread): J = 16 serves n <= 8192
 // (128 columns, four CTAs per SM), J = 32 serves n <= 16384 (256 columns, two
 // CTAs per SM, where the fields in shared memory leave one).
@@ -703,6 +709,64 @@ __device__ __forceinline__ double tm_ld_f64(uint32_t taddr) {
   return __hiloint2double((int)hi, (int)lo);
 }
 
+// A float weight as float64, scaled by 2^-896: its bits moved into the wider
+// fields (exact for every finite weight, zeros and denormals included), three
+// integer operations in place of a conversion, which runs at a quarter of the
+// float64 rate. A coefficient +-2 x 2^896 undoes the scale inside the exact
+// product of a multiply-add, so the sum is the same number.
+__device__ __forceinline__ double weight_scaled(float w) {
+  const int b = __float_as_int(w);
+  return __hiloint2double((b >> 3) & (int)0x8FFFFFFF, b << 29);
+}
+constexpr double kUnscale2 = 0x1p897;  // 2 / (the scale of weight_scaled)
+
+// Reference nodes of a float search: nodes whose gains are known to bound the
+// selection from below, one per warp of the CTA, kept alike in every thread.
+// The largest gain after a flip is at least a reference's own new gain, its gain
+// before +- 2 W; the margin covers the roundings of the float gain and of this
+// sum and one float's spacing, so a node whose float64 gain is below the bound
+// has a float gain below the largest and cannot be the selection, ties included.
+// A warp's best node, where it reached the bound, becomes its reference.
+template <int R>
+struct GainRefs {
+  float g[R];     // lower bound of the gain; -inf: none
+  uint32_t v[R];  // node << 1 | its bit
+
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      g[i] = -INFINITY;
+      v[i] = 0u;
+    }
+  }
+  // The references' weights in row `row` (of the node flipped next).
+  __device__ __forceinline__ void load(const float* __restrict__ row, float (&w)[R]) const {
+#pragma unroll
+    for (int i = 0; i < R; ++i) w[i] = __ldg(row + (v[i] >> 1));
+  }
+  // After flipping k (bit xk), w the references' weights to it: the high word
+  // that every gain reaching the bound has at least (as signed integers; INT_MIN
+  // while the bound is not well above zero, when every gain is looked at).
+  __device__ __forceinline__ int flip(const float (&w)[R], int k, int xk) {
+    float bound = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float w2 = 2.0f * w[i];
+      const float d = (int)(v[i] & 1u) == xk ? -w2 : w2;
+      const float ng = g[i] + d - (fabsf(g[i]) + fabsf(w2)) * 9.5367431640625e-07f;  // 2^-20
+      g[i] = (int)(v[i] >> 1) == k ? -INFINITY : ng;
+      bound = fmaxf(bound, g[i]);
+    }
+    return bound > 1e-30f ? (__float_as_int(bound) >> 3) + 0x38000000 : INT_MIN;
+  }
+  __device__ __forceinline__ void found(int i, unsigned long long key) {
+    if (key != 0ull) {
+      g[i] = unord_f32((uint32_t)(key >> 32));
+      v[i] = (0x3FFFFFFFu - ((uint32_t)key >> 1)) << 1 | ((uint32_t)key & 1u);
+    }
+  }
+};
+
 struct TmCtx {
   const float* W;
   int n, ld;
@@ -711,75 +775,125 @@ struct TmCtx {
   uint32_t tbase;      // this warp's lanes, column 0 of the CTA's allocation
 };
 
-// One flip pass of the TMEM form: with k >= 0 the row k is in the stage,
-// flip k (coefficient -2 x_k) in this thread's fields and bits, and return in
-// *out_gk the exact gain of k before the flip (its field is unchanged by its
-// own flip, W_kk = 0: the owner warp reads it back once instead of every
-// thread keeping the field of its best node); then the CTA's best key.
-template <bool UPD, int J>
-__device__ __forceinline__ void tm_pass(const TmCtx& c, int k, int xk,
-                                        unsigned long long (*red_key)[4], double* s_yk, int par,
-                                        unsigned long long* out_key, double* out_gk) {
-  const int t = threadIdx.x, n = c.n;
-  const double coef = xk ? -2.0 : 2.0;
+// One flip pass of the TMEM form: with UPD the row k is on its way to the stage,
+// 2048 nodes per mbarrier, and each chunk is waited for when it is needed; flip k
+// (coefficient -2 x_k) in this thread's fields and bits, then the CTA's best key
+// and the exact gain of its node. KICK: k was not the selection; *out_gk is then
+// its gain before the flip (its field is unchanged by its own flip, W_kk = 0).
+// xm: the bits of this thread's nodes (node 4 t + 512 j + i: bit 4 j + i).
+// The selection compares float gains, but a float64 gain is only converted when
+// it reaches the references' bound: a pass then has a handful of conversions
+// instead of two per node, which bound it (16 lanes per clock per SM).
+template <bool UPD, bool KICK, int J>
+__device__ __forceinline__ void tm_pass(const TmCtx& c, int k, int xk, uint32_t (&xm)[J / 8], GainRefs<4>& refs,
+                                        const float (&rw)[4], uint64_t* bars, uint32_t phase, int* s_fail,
+                                        unsigned long long (*red_key)[4], double (*red_g)[4], double* s_yk, int par,
+                                        unsigned long long* out_key, double* out_g, double* out_gk) {
+  const int t = threadIdx.x, n = c.n, lane = t & 31, warp = t >> 5;
+  const double coef = xk ? -kUnscale2 : kUnscale2;
   float bv = -INFINITY;
-  int bi = -1;
+  uint32_t bn = 0xFFFFFFFFu;  // best node << 1 | bit
+  double bg = 0.0;
+  int hbound = INT_MIN;
+  tm_wait_st();  // the pass before's fields
+  if (UPD) {
+    const int owner = (k >> 2) & (TM_BT - 1);
+    if (KICK && warp == owner >> 5) {
+      const double y = tm_ld_f64(c.tbase + 2u * (uint32_t)(4 * (k / 512) + (k & 3)));
+      if (lane == (owner & 31)) s_yk[par] = xk ? y : -y;
+    }
+    if (owner == t) {  // the owner toggles bit k
+      c.bits[k >> 5] ^= 1u << (k & 31);
+      const int e = 4 * (k / 512) + (k & 3);
+#pragma unroll
+      for (int q = 0; q < J / 8; ++q)
+        if ((e >> 5) == q) xm[q] ^= 1u << (e & 31);
+    }
+    hbound = refs.flip(rw, k, xk);
+  }
 #pragma unroll 1
   for (int q = 0; q < J / 4; ++q) {
     if (2048 * q >= n) break;  // (uniform: no node of this chunk below n)
     uint32_t r[32];
     tc::tmem_load32(c.tbase + 32u * q, r);
+    // the chunk's 16 bits, in the high half (selected without indexing)
+    uint32_t m16 = 0;
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int v0 = 4 * t + 512 * (4 * q + jj);
-      if (v0 >= n) continue;
-      float w4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      if (UPD) {
-        const float4 s4 = *reinterpret_cast<const float4*>(c.stage + v0);
-        w4[0] = s4.x; w4[1] = s4.y; w4[2] = s4.z; w4[3] = s4.w;
-        if ((unsigned)(k - v0) < 4u) c.bits[k >> 5] ^= 1u << (k & 31);
+    for (int h = 0; h < J / 8; ++h)
+      if ((q >> 1) == h) m16 = (q & 1) ? xm[h] : xm[h] << 16;
+    m16 = ~m16;  // set: bit 0, the gain is -field
+    const int v0 = 4 * t + 2048 * q;
+    // All 16 nodes without a branch: chains of a few dependent operations that
+    // overlap (a branch per group of four ran them one after the other, 70
+    // cycles per node). Nodes at and past n update fields that nothing reads.
+    if (UPD) {
+      if (!tc::mbar_wait_spin(&bars[q], (phase >> q) & 1u)) *s_fail = 1;  // this chunk of the row
+      float4 s4[4];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) s4[jj] = *reinterpret_cast<const float4*>(c.stage + v0 + 512 * jj);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float w = (e & 3) == 0 ? s4[e >> 2].x : (e & 3) == 1 ? s4[e >> 2].y : (e & 3) == 2 ? s4[e >> 2].z : s4[e >> 2].w;
+        const double y = fma(coef, weight_scaled(w), __hiloint2double((int)r[2 * e + 1], (int)r[2 * e]));
+        r[2 * e] = (uint32_t)__double2loint(y);
+        r[2 * e + 1] = (uint32_t)__double2hiint(y);
       }
-      const uint32_t nib = c.bits[v0 >> 5] >> (v0 & 31);
-      const bool full = v0 + 3 < n;
+    }
+    // For a positive bound a gain that reaches it has at least its high word
+    // (as signed integers; negative gains are negative).
+    auto gain_hi = [&](int e) { return (int)(r[2 * e + 1] ^ ((m16 << (15 - e)) & 0x80000000u)); };
+    int top[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (full || v0 + i < n) {
-          const int s = 8 * jj + 2 * i;
-          double y = __hiloint2double((int)r[s + 1], (int)r[s]);
-          if (UPD) {
-            y += coef * (double)w4[i];
-            r[s] = (uint32_t)__double2loint(y);
-            r[s + 1] = (uint32_t)__double2hiint(y);
-          }
-          const float yf = (float)y;
-          const float gv = ((nib >> i) & 1u) ? yf : -yf;
-          if (gv > bv) {
-            bv = gv;
-            bi = v0 + i;
-          }
+    for (int jj = 0; jj < 4; ++jj)
+      top[jj] = max(max(gain_hi(4 * jj), gain_hi(4 * jj + 1)), max(gain_hi(4 * jj + 2), gain_hi(4 * jj + 3)));
+    if (max(max(top[0], top[1]), max(top[2], top[3])) >= hbound) {
+      // (rare: opaque copies keep its index arithmetic out of the main path)
+      int vq = v0;
+      uint32_t mq = m16;
+      asm volatile("" : "+r"(vq), "+r"(mq));
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        if (top[jj] < hbound) continue;
+        double g[4];
+        float gf[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          g[i] = __hiloint2double(gain_hi(4 * jj + i), (int)r[2 * (4 * jj + i)]);
+          gf[i] = (float)g[i];
+        }
+        // (selects, no branches: nodes below the bound cannot win either way)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int v = vq + 512 * jj + i;
+          const bool up = v < n && gf[i] > bv;  // v ascends: strict '>' keeps the lowest node
+          bv = up ? gf[i] : bv;
+          bg = up ? g[i] : bg;
+          bn = up ? (uint32_t)v << 1 | (((mq >> (16 + 4 * jj + i)) & 1u) ^ 1u) : bn;
         }
       }
     }
     if (UPD) tm_st32(c.tbase + 32u * q, r);
   }
-  const int lane = t & 31, warp = t >> 5;
-  if (UPD) {
-    tm_wait_st();
-    const int owner = (k >> 2) & (TM_BT - 1);
-    if (warp == owner >> 5) {
-      const double y = tm_ld_f64(c.tbase + 2u * (uint32_t)(4 * (k / 512) + (k & 3)));
-      if (lane == (owner & 31)) s_yk[par] = y;
-    }
-  }
-  const int bx = bi >= 0 ? (int)((c.bits[bi >> 5] >> (bi & 31)) & 1u) : 0;
-  const unsigned long long key = bi >= 0 ? bkey(bv, bi, bx) : 0ull;
+  const unsigned long long key = bn != 0xFFFFFFFFu ? bkey(bv, (int)(bn >> 1), (int)(bn & 1u)) : 0ull;
   const unsigned long long wk = bmax_key(key);
-  const uint32_t src = __ballot_sync(0xFFFFFFFFu, key == wk && wk != 0ull);
-  if (lane == (src ? __ffs(src) - 1 : 0)) red_key[par][warp] = wk;
+  if (wk != 0ull ? key == wk : lane == 0) {
+    red_key[par][warp] = wk;
+    red_g[par][warp] = bg;
+  }
   __syncthreads();
-  const unsigned long long sk = lane < 4 ? red_key[par][lane] : 0ull;
-  *out_key = bmax_key(sk);
-  if (UPD) *out_gk = xk ? s_yk[par] : -s_yk[par];
+  unsigned long long bk = 0ull;
+  double g = 0.0;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    const unsigned long long o = red_key[par][w];
+    const double og = red_g[par][w];
+    refs.found(w, o);
+    g = o > bk ? og : g;
+    bk = o > bk ? o : bk;
+  }
+  *out_key = bk;
+  *out_g = g;
+  if (KICK) *out_gk = s_yk[par];
 }
 
 template <int J>
@@ -793,8 +907,10 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
   extern __shared__ __align__(16) unsigned char tm_smem[];
   __shared__ double red[4];
   __shared__ unsigned long long red_key[2][4];
+  __shared__ double red_g[2][4];
   __shared__ double s_yk[2];
-  __shared__ __align__(8) uint64_t row_bar;
+  __shared__ int s_fail;
+  __shared__ __align__(8) uint64_t row_bar[J / 4];  // one per 2048 nodes of the row
   __shared__ uint32_t s_tmem;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   float* stage = reinterpret_cast<float*>(tm_smem);
@@ -809,13 +925,14 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (t == 0) {
-    tc::mbar_init(&row_bar, 1);
+    s_fail = 0;
+    for (int q = 0; q < J / 4; ++q) tc::mbar_init(&row_bar[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  uint32_t phase = 0;
+  uint32_t phase = 0;  // bit q: parity of row_bar[q]
   bool failed = false;
   for (int task = blockIdx.x; task < tasks && !failed; task += gridDim.x) {
     const BatchGraph G = graphs[task_graph[task]];
@@ -834,6 +951,16 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
     // summed over the node's row list), stored to TMEM 16 nodes at a time;
     // x_v y_v into this thread's share of q = x^T W x
     double qpart = 0.0;
+    uint32_t xm[J / 8];  // this thread's bits: node 4 t + 512 j + i at 4 j + i
+#pragma unroll
+    for (int q = 0; q < J / 8; ++q) {
+      xm[q] = 0u;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int v = 4 * t + 512 * (8 * q + j);
+        if (v < n) xm[q] |= ((bits[v >> 5] >> (v & 31)) & 15u) << (4 * j);
+      }
+    }
     const double* __restrict__ yrow =
         (start_fields && !G.adj_ptr) ? start_fields + (size_t)task * fields_pitch : nullptr;
 #pragma unroll 1
@@ -873,34 +1000,35 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
     unsigned long long nflips = 0;
     int timeout = 0;
     unsigned long long key;
-    double gflip = 0.0;  // the gain of the node the last pass flipped, before the flip
+    double gsel = 0.0;  // the exact gain of the selected node
+    double gflip = 0.0; // the gain of a kicked node before its flip
     int par = 0;
-    // the row of node k into the stage by one bulk copy (every thread has
-    // finished reading the previous row: the pass before ended on a CTA
-    // barrier)
-    auto flip = [&](int k, int xk) -> bool {
+    GainRefs<4> refs;
+    refs.clear();
+    const uint32_t used = (1u << ((n + 2047) / 2048)) - 1u;  // the row's chunks
+    // The row of node k into the stage, a bulk copy per 2048 nodes (every thread
+    // has finished reading the previous row: the pass before ended on a CTA
+    // barrier). The pass's threads wait for the copies themselves (bounded); a
+    // wait that runs out anywhere raises a flag that all read behind the pass's
+    // barrier, so it stops the task everywhere.
+    float rw[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // the references' weights to k
+    auto fetch = [&](int k) {
+      const float* row = c.W + (size_t)k * c.ld;
+      refs.load(row, rw);
       if (t == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const uint32_t bytes = (uint32_t)(((n + 3) & ~3) * 4);
-        tc::mbar_expect_tx(&row_bar, bytes);
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                tc::smem_u32(stage)),
-            "l"(c.W + (size_t)k * c.ld), "r"(bytes), "r"(tc::smem_u32(&row_bar))
-            : "memory");
+        for (int q = 0; 2048 * q < n; ++q) {
+          const uint32_t bytes = (uint32_t)(min(2048, ((n + 3) & ~3) - 2048 * q) * 4);
+          tc::mbar_expect_tx(&row_bar[q], bytes);
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  tc::smem_u32(stage + 2048 * q)),
+              "l"(row + 2048 * q), "r"(bytes), "r"(tc::smem_u32(&row_bar[q]))
+              : "memory");
+        }
       }
-      // (one lane per warp waits, bounded; the CTA then agrees, so a wait
-      // that ran out anywhere stops the task everywhere)
-      bool ok = true;
-      if (lane == 0) ok = tc::mbar_wait_spin(&row_bar, phase);
-      ok = __syncthreads_and(ok ? 1 : 0) != 0;
-      phase ^= 1u;
-      if (!ok) return false;
-      tm_pass<true, J>(c, k, xk, red_key, s_yk, par, &key, &gflip);
-      par ^= 1;
-      return true;
     };
-    tm_pass<false, J>(c, -1, 0, red_key, s_yk, par, &key, &gflip);
+    tm_pass<false, false, J>(c, -1, 0, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel, &gflip);
     par ^= 1;
     for (int r = 0; r <= rounds && !failed; ++r) {
       for (int f = 0;; ++f) {
@@ -911,12 +1039,17 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         }
         const int k = (int)(0x3FFFFFFFu - (((uint32_t)key) >> 1));
         const int xk = (int)(key & 1ull);
-        if (!flip(k, xk)) {
+        fetch(k);
+        val += scale * gsel;
+        tm_pass<true, false, J>(c, k, xk, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel,
+                                &gflip);
+        par ^= 1;
+        phase ^= used;
+        ++nflips;
+        if (s_fail) {
           failed = true;
           break;
         }
-        val += scale * gflip;
-        ++nflips;
       }
       if (failed) break;
       if (val > best) {
@@ -937,12 +1070,17 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         const int xp = (bits[pick >> 5] >> (pick & 31)) & 1;
         __syncthreads();  // everyone has read bit and kicked set before they change
         if (t == 0) kicked[pick >> 5] |= 1u << (pick & 31);
-        if (!flip(pick, xp)) {
+        fetch(pick);
+        tm_pass<true, true, J>(c, pick, xp, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel,
+                               &gflip);
+        par ^= 1;
+        phase ^= used;
+        val += scale * gflip;  // float64 gain of the kicked node
+        ++nflips;
+        if (s_fail) {
           failed = true;
           break;
         }
-        val += scale * gflip;  // float64 gain of the kicked node
-        ++nflips;
       }
     }
     if (t == 0) {
