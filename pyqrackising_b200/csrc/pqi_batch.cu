@@ -298,6 +298,17 @@ __device__ __forceinline__ void flip_and_select(const TaskCtx<WT, GT>& c, int k,
   }
 }
 
+// A float weight as float64, scaled by 2^-896: its bits moved into the wider
+// fields (exact for every finite weight, zeros and denormals included), three
+// integer operations in place of a conversion, which runs at a quarter of the
+// float64 rate. A coefficient +-2 x 2^896 undoes the scale inside the exact
+// product of a multiply-add, so the sum is the same number.
+__device__ __forceinline__ double weight_scaled(float w) {
+  const int b = __float_as_int(w);
+  return __hiloint2double((b >> 3) & (int)0x8FFFFFFF, b << 29);
+}
+constexpr double kUnscale2 = 0x1p897;  // 2 / (the scale of weight_scaled)
+
 // Starting local fields of many tasks at once, for graphs without row lists:
 // Y[t][v] = sum_u x_tu W[u][v] (x = +-1), u ascending from 0 - the order and
 // the accumulation type (float64 for float weights, int32 for int8) of the
@@ -650,6 +661,298 @@ __global__ void __launch_bounds__(BT, (F32 ? 4 : 3) * 256 / BT) batch_search_ker
 }
 
 // ---------------------------------------------------------------------------
+// Register form of the CTA search, for graphs of at most 4 NG BT nodes (and
+// float64 or int32 fields): thread t owns the nodes v = 4 t + 4 BT j + i (j < NG)
+// and keeps their fields and bits in registers, so a flip is one vector load
+// per group, the updates and a branch-free selection in registers, the warps'
+// bests (key and exact gain) through shared memory and one barrier. The search,
+// the selection rule, the kick stream and the float64 values are those of
+// batch_search_kernel, which moves every field through shared memory behind
+// branches (300 instructions per warp and flip at 8 nodes per thread). Shared
+// memory keeps a copy of the bits for kicks and results. Bound by the row load
+// and the selection's dependency chain where few tasks are resident, by issue
+// where many are; a selection as a tree over the 4 NG nodes spills and was 8 %
+// slower, and 20 % more resident threads at fewer registers up to 10 %.
+//
+// Tasks come from a queue, largest graphs first, when there are more of them
+// than CTAs: tasks differ in length by more than ten, and with a fixed share per
+// CTA a quarter of the launch waited for the last ones. 48 float (int) graphs of
+// 64 to 1024 nodes, 16 starts each, 4 rounds: 3.83 (2.17) ms -> 2.00 (1.23).
+template <typename WT>
+struct RegField {
+  typedef double type;
+};
+template <>
+struct RegField<int8_t> {
+  typedef int type;
+};
+
+// Minimum resident threads per SM the register budget is sized for.
+template <typename WT>
+constexpr int reg_threads(int NG) {
+  return sizeof(WT) == 1 ? (NG == 1 ? 1536 : NG == 2 ? 1280 : 896) : (NG == 1 ? 1024 : NG == 2 ? 768 : 512);
+}
+
+template <bool UPD, bool KICK, typename WT, int NG, int BT>
+__device__ __forceinline__ void reg_pass(const WT* __restrict__ W, int ld, int n, int k, int xk,
+                                         typename RegField<WT>::type (&y)[4 * NG], uint32_t& xm, uint32_t* bits,
+                                         unsigned long long (*red_key)[BT / 32], double (*red_g)[BT / 32],
+                                         double* s_gk, int par, unsigned long long* out_key, double* out_g,
+                                         double* out_gk) {
+  typedef typename RegField<WT>::type GT;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  unsigned long long key = 0ull;
+  GT bg = 0;
+  if (4 * (t & ~31) < n) {  // (a warp without nodes only waits)
+    if constexpr (UPD) {
+      const WT* __restrict__ row = W + (size_t)k * ld;
+      WT w[4 * NG];
+#pragma unroll
+      for (int j = 0; j < NG; ++j) {
+        const int v = 4 * t + 4 * BT * j;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[4 * j + i] = (WT)0;
+        if (v < n) {  // (rows are zero padded to a multiple of 128)
+          if constexpr (sizeof(WT) == 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(row + v));
+            w[4 * j] = q.x; w[4 * j + 1] = q.y; w[4 * j + 2] = q.z; w[4 * j + 3] = q.w;
+          } else {
+            const char4 q = __ldg(reinterpret_cast<const char4*>(row + v));
+            w[4 * j] = q.x; w[4 * j + 1] = q.y; w[4 * j + 2] = q.z; w[4 * j + 3] = q.w;
+          }
+        }
+      }
+      if (t == ((k >> 2) & (BT - 1))) {  // k's owner
+        const int e = 4 * (k / (4 * BT)) + (k & 3);
+        if constexpr (KICK) {
+          // its gain before the flip (W_kk = 0: its field does not change)
+          GT yk = y[0];
+#pragma unroll
+          for (int q = 1; q < 4 * NG; ++q) yk = e == q ? y[q] : yk;
+          s_gk[par] = xk ? (double)yk : -(double)yk;
+        }
+        xm ^= 1u << e;
+        bits[k >> 5] ^= 1u << (k & 31);
+      }
+#pragma unroll
+      for (int e = 0; e < 4 * NG; ++e) {
+        if constexpr (sizeof(WT) == 4) {
+          y[e] = fma(xk ? -kUnscale2 : kUnscale2, weight_scaled(w[e]), y[e]);
+        } else {
+          y[e] += xk ? -2 * (int)w[e] : 2 * (int)w[e];
+        }
+      }
+    }
+    // the thread's best: float gain (exact for int fields below 2^24), then the
+    // lowest node; v ascends with e, so strict '>' keeps it, and NaN never wins
+    float bv = -INFINITY;
+    uint32_t bn = 0xFFFFFFFFu;  // node << 1 | bit
+#pragma unroll
+    for (int e = 0; e < 4 * NG; ++e) {
+      const int v = 4 * t + 4 * BT * (e >> 2) + (e & 3);
+      const uint32_t xv = (xm >> e) & 1u;
+      GT g;
+      if constexpr (sizeof(WT) == 4) {
+        g = __hiloint2double(__double2hiint(y[e]) ^ (int)(xv ? 0u : 0x80000000u), __double2loint(y[e]));
+      } else {
+        g = xv ? y[e] : -y[e];
+      }
+      const float gf = (float)g;
+      const bool up = v < n && gf > bv;
+      bv = up ? gf : bv;
+      bg = up ? g : bg;
+      bn = up ? (uint32_t)v << 1 | xv : bn;
+    }
+    if (bn != 0xFFFFFFFFu) key = bkey(bv, (int)(bn >> 1), (int)(bn & 1u));
+  }
+  const unsigned long long wk = bmax_key(key);
+  if (wk != 0ull ? key == wk : lane == 0) {
+    red_key[par][warp] = wk;
+    red_g[par][warp] = (double)bg;
+  }
+  __syncthreads();
+  constexpr int NW = BT / 32;
+  unsigned long long bk[NW];
+  int bw[NW];
+#pragma unroll
+  for (int q = 0; q < NW; ++q) {
+    bk[q] = red_key[par][q];
+    bw[q] = q;
+  }
+#pragma unroll
+  for (int d = 1; d < NW; d *= 2)
+#pragma unroll
+    for (int q = 0; q < NW; q += 2 * d) {
+      const bool up = bk[q + d] > bk[q];
+      bk[q] = up ? bk[q + d] : bk[q];
+      bw[q] = up ? bw[q + d] : bw[q];
+    }
+  *out_key = bk[0];
+  *out_g = red_g[par][bw[0]];
+  if constexpr (KICK) *out_gk = s_gk[par];
+}
+
+template <typename WT, int NG, int BT>
+__global__ void __launch_bounds__(BT, reg_threads<WT>(NG) / BT) batch_reg_kernel(
+    const BatchGraph* __restrict__ graphs, const int* __restrict__ task_graph,
+    const uint32_t* __restrict__ init_states, int words_pitch, int tasks, int spin, int rounds,
+    int kick, int flip_budget, uint64_t seed, const double* __restrict__ kick_cdf,
+    const long long* __restrict__ cdf_offset, uint32_t* __restrict__ best_states,
+    double* __restrict__ best_values, unsigned long long* __restrict__ flips_total,
+    int* __restrict__ status, const double* __restrict__ start_fields, int fields_pitch,
+    const int* __restrict__ order, int* __restrict__ queue) {
+  typedef typename RegField<WT>::type GT;
+  constexpr int NW = BT / 32;
+  __shared__ GT y0[4 * BT * NG];  // starting fields in node order
+  __shared__ uint32_t bits[4 * BT * NG / 32], kicked[4 * BT * NG / 32];
+  __shared__ unsigned long long red_key[2][NW];
+  __shared__ double red_g[2][NW];
+  __shared__ double s_gk[2];
+  __shared__ double red[NW];
+  __shared__ int s_task;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int q = blockIdx.x;; q += gridDim.x) {
+    if (queue) {
+      if (t == 0) s_task = atomicAdd(queue, 1);
+      __syncthreads();
+      q = s_task;
+    }
+    if (q >= tasks) break;
+    const int task = order ? order[q] : q;
+    const BatchGraph G = graphs[task_graph[task]];
+    const int n = G.n, n32 = (n + 31) >> 5;
+    const WT* __restrict__ W = static_cast<const WT*>(G.W);
+    uint32_t* best_bits = best_states + (size_t)task * words_pitch;
+    for (int w = t; w < n32; w += BT) bits[w] = init_states[(size_t)task * words_pitch + w];
+    __syncthreads();
+    // 1. starting fields (from the start pass, or summed over the node's row list
+    // in column order), x_v y_v into q = x^T W x in batch_search_kernel's order,
+    // and then the own nodes' fields and bits
+    const double* __restrict__ yrow = G.adj_ptr ? nullptr : start_fields + (size_t)task * fields_pitch;
+    double qpart = 0.0;
+    for (int v = t; v < n; v += BT) {
+      GT acc = 0;
+      if (yrow) {
+        acc = (GT)yrow[v];
+      } else {
+        const long long e1 = G.adj_ptr[v + 1];
+        for (long long a = G.adj_ptr[v]; a < e1; ++a) {
+          const int u = G.adj_col[a];
+          if (u == v) continue;
+          const GT w = (GT)G.adj_val[a];
+          acc += ((bits[u >> 5] >> (u & 31)) & 1) ? w : -w;
+        }
+      }
+      y0[v] = acc;
+      qpart += ((bits[v >> 5] >> (v & 31)) & 1) ? (double)acc : -(double)acc;
+    }
+    for (int o = 16; o > 0; o >>= 1) qpart += __shfl_xor_sync(0xFFFFFFFFu, qpart, o);
+    if (lane == 0) red[warp] = qpart;
+    __syncthreads();
+    GT y[4 * NG];
+    uint32_t xm = 0;
+#pragma unroll
+    for (int e = 0; e < 4 * NG; ++e) {
+      const int v = 4 * t + 4 * BT * (e >> 2) + (e & 3);
+      y[e] = v < n ? y0[v] : (GT)0;
+      if (v < n) xm |= ((bits[v >> 5] >> (v & 31)) & 1u) << e;
+    }
+    double qv = 0.0;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) qv += red[i];
+    const double scale = spin ? 2.0 : 1.0;
+    double val = spin ? -qv / 2.0 : (2.0 * G.upper_sum - qv) / 4.0;
+    double best = -INFINITY;
+    unsigned long long nflips = 0;
+    int timeout = 0;
+    unsigned long long key;
+    double gsel = 0.0, gkick = 0.0;  // exact gains: the selection's, a kicked node's
+    int par = 0;
+    reg_pass<false, false, WT, NG, BT>(W, G.ld, n, 0, 0, y, xm, bits, red_key, red_g, s_gk, par, &key, &gsel, &gkick);
+    par ^= 1;
+    for (int r = 0; r <= rounds; ++r) {
+      // steepest ascent: flip the best node while its gain is positive
+      for (int f = 0;; ++f) {
+        if (key == 0ull || !(unord_f32((uint32_t)(key >> 32)) > 0.0f)) break;
+        if (f >= flip_budget) {
+          timeout = 1;
+          break;
+        }
+        val += scale * gsel;
+        reg_pass<true, false, WT, NG, BT>(W, G.ld, n, (int)(0x3FFFFFFFu - (((uint32_t)key) >> 1)), (int)(key & 1ull), y,
+                                          xm, bits, red_key, red_g, s_gk, par, &key, &gsel, &gkick);
+        par ^= 1;
+        ++nflips;
+      }
+      if (val > best) {
+        best = val;
+        for (int w = t; w < n32; w += BT) best_bits[w] = bits[w];
+      }
+      if (r == rounds) break;
+      // kicks, without replacement within the round (as batch_search_kernel)
+      for (int w = t; w < n32; w += BT) kicked[w] = 0u;
+      __syncthreads();
+      for (int j = 0; j < kick; ++j) {
+        int pick = 0;
+        for (int attempt = 0; attempt < 16; ++attempt) {
+          const double u =
+              bunif(seed, (uint64_t)task * 1315423911ull + r, (uint64_t)j + ((uint64_t)attempt << 20));
+          pick = draw_node(u, n, kick_cdf ? kick_cdf + cdf_offset[task_graph[task]] : nullptr);
+          if (!((kicked[pick >> 5] >> (pick & 31)) & 1u)) break;
+        }
+        const int xp = (bits[pick >> 5] >> (pick & 31)) & 1;
+        __syncthreads();  // everyone has read bit and kicked set before they change
+        if (t == 0) kicked[pick >> 5] |= 1u << (pick & 31);
+        reg_pass<true, true, WT, NG, BT>(W, G.ld, n, pick, xp, y, xm, bits, red_key, red_g, s_gk, par, &key, &gsel,
+                                         &gkick);
+        par ^= 1;
+        val += scale * gkick;
+        ++nflips;
+      }
+    }
+    if (t == 0) {
+      best_values[task] = best;
+      atomicAdd(flips_total, nflips);
+      if (timeout) atomicExch(status, PQI_ETIMEOUT);
+    }
+    __syncthreads();
+  }
+}
+
+// The tasks in order of decreasing graph size (in 256 classes) and the queue's
+// counter, one block.
+__global__ void __launch_bounds__(1024) task_order_kernel(const BatchGraph* __restrict__ graphs,
+                                                          const int* __restrict__ task_graph, int tasks, int max_n,
+                                                          int* __restrict__ order, int* __restrict__ queue) {
+  __shared__ int at[256];
+  if (threadIdx.x < 256) at[threadIdx.x] = 0;
+  if (threadIdx.x == 0) *queue = 0;
+  __syncthreads();
+  auto cls = [&](int q) {
+    return 255 - min(255, (int)((long long)graphs[task_graph[q]].n * 256 / (max_n + 1)));
+  };
+  for (int q = threadIdx.x; q < tasks; q += blockDim.x) atomicAdd(&at[cls(q)], 1);
+  __syncthreads();
+  if (threadIdx.x < 32) {  // exclusive scan of the classes, eight per lane
+    int c[8], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      c[i] = sum;
+      sum += at[8 * threadIdx.x + i];
+    }
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int z = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if ((int)threadIdx.x >= o) incl += z;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) at[8 * threadIdx.x + i] = incl - sum + c[i];
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < tasks; q += blockDim.x) order[atomicAdd(&at[cls(q)], 1)] = q;
+}
+
+// ---------------------------------------------------------------------------
 // Float64 local fields in tensor memory (float weights, 4096 < n <= 16384).
 //
 // The shared-memory form holds a task's float64 fields in shared memory:
@@ -708,17 +1011,6 @@ __device__ __forceinline__ double tm_ld_f64(uint32_t taddr) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
   return __hiloint2double((int)hi, (int)lo);
 }
-
-// A float weight as float64, scaled by 2^-896: its bits moved into the wider
-// fields (exact for every finite weight, zeros and denormals included), three
-// integer operations in place of a conversion, which runs at a quarter of the
-// float64 rate. A coefficient +-2 x 2^896 undoes the scale inside the exact
-// product of a multiply-add, so the sum is the same number.
-__device__ __forceinline__ double weight_scaled(float w) {
-  const int b = __float_as_int(w);
-  return __hiloint2double((b >> 3) & (int)0x8FFFFFFF, b << 29);
-}
-constexpr double kUnscale2 = 0x1p897;  // 2 / (the scale of weight_scaled)
 
 // Reference nodes of a float search: nodes whose gains are known to bound the
 // selection from below, one per warp of the CTA, kept alike in every thread.
@@ -1440,6 +1732,43 @@ static pqi_status batch_search_impl(const void* graphs, int num_graphs, const in
       PQI_TRY(cudaFreeAsync(sf, s));
       return PQI_OK;
     }
+  }
+  // Fields in registers where a thread's groups are at most four (float64 or
+  // int32 fields, starting fields at hand). Against shared memory, 256 / 128 /
+  // 64 threads per task, ms (4 rounds of n/64 kicks, dense float graphs): n = 500
+  // x 2000 tasks 1.51 / 1.02 / 0.95 -> 1.30 / 0.80 / 0.64, n = 1000 x 1200 2.34 /
+  // 1.80 / 1.62 -> 2.32 / 1.43 / 1.19, n = 2047 x 500 3.69 / 3.10 -> 2.97 / 2.16,
+  // n = 4096 x 148 6.03 -> 3.38. Eight groups would need 255 registers a thread.
+  if ((i8 || !f32) && sf && groups <= 4) {
+    const int NG = groups <= 1 ? 1 : groups <= 2 ? 2 : 4;
+    auto launch = [&](auto kern) -> pqi_status {
+      PQI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, 0));
+      const int grid = std::max(1, std::min(tasks, num_sms * std::max(1, per_sm)));
+      int* queue = nullptr;
+      if (tasks > grid &&  // (freed behind the search, on its stream; fixed shares without it)
+          cudaMallocAsync(reinterpret_cast<void**>(&queue), ((size_t)tasks + 1) * sizeof(int), s) != cudaSuccess) {
+        (void)cudaGetLastError();
+        queue = nullptr;
+      }
+      if (queue) {
+        task_order_kernel<<<1, 1024, 0, s>>>(gd, task_graph, tasks, max_n, queue + 1, queue);
+        PQI_LAUNCHED("task_order_kernel");
+      }
+      kern<<<grid, bt, 0, s>>>(gd, task_graph, init_states, words_pitch, tasks, is_spin_glass, rounds, kick,
+                               flip_budget, seed, kick_cdf, cdf_offset, best_states, best_values, flips_total, status,
+                               sf, sf_pitch, queue ? queue + 1 : nullptr, queue);
+      PQI_LAUNCHED("batch_reg_kernel");
+      if (queue) PQI_TRY(cudaFreeAsync(queue, s));
+      PQI_TRY(cudaFreeAsync(sf, s));
+      return PQI_OK;
+    };
+#define PQI_REG(WT_, BT_)                                  \
+  (NG == 1   ? launch(batch_reg_kernel<WT_, 1, BT_>)       \
+   : NG == 2 ? launch(batch_reg_kernel<WT_, 2, BT_>)       \
+             : launch(batch_reg_kernel<WT_, 4, BT_>))
+    if (i8) return bt == 64 ? PQI_REG(int8_t, 64) : bt == 128 ? PQI_REG(int8_t, 128) : PQI_REG(int8_t, 256);
+    return bt == 64 ? PQI_REG(float, 64) : bt == 128 ? PQI_REG(float, 128) : PQI_REG(float, 256);
+#undef PQI_REG
   }
   // row loads per thread: groups of four nodes, CH groups in flight per chunk
   // (the whole row for n <= 4 * 256 * CH). CH = 4 keeps three CTAs per SM
