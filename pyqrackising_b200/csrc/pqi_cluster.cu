@@ -12,6 +12,9 @@
 //      (y_v += coef * W_kv, one float4 / char4 of row k per group; the owner of
 //      k toggles its bit) and folds the new gains g_v = x_v y_v into a local
 //      argmax: float gain first, then the lowest node (a 64-bit key);
+//      (branch-free; with it and a row prefetch only for candidates that change,
+//      n = 6000 int8, 20 tasks on clusters of 8, went from 4.47 to 3.71 ms and
+//      n = 8192 float, 8 tasks, from 6.98 to 6.06, 5.38 with the loads of kAhead);
 //   2. warp maxima (two 32-bit redux steps) meet in shared memory behind the
 //      flip's one CTA barrier; warp 0 reduces them and its lanes 0..C-1 write the
 //      CTA's best (key, exact gain) into slot [rank] of every CTA with st.async,
@@ -84,8 +87,41 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long ke
   return ((unsigned long long)hi << 32) | lo;
 }
 
+// The thread's groups of row k (slice from node lo; group j at lo + 4 (t + T j)).
+// Volatile, so that the loads ahead of their use are issued where they stand.
 template <typename WT, int NG>
-__global__ void __launch_bounds__(256) cluster_ascent_kernel(
+__device__ __forceinline__ void load_row(const WT* __restrict__ row, int v0, int step, int n, WT (&w)[4 * NG]) {
+#pragma unroll
+  for (int j = 0; j < NG; ++j) {
+    const int v = v0 + step * j;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[4 * j + i] = (WT)0;
+    if (v < n) {  // (rows are zero padded to a multiple of 128)
+      if constexpr (sizeof(WT) == 4) {
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(w[4 * j]), "=f"(w[4 * j + 1]), "=f"(w[4 * j + 2]), "=f"(w[4 * j + 3])
+                     : "l"(row + v));
+      } else {
+        uint32_t q;
+        asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(q) : "l"(row + v));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[4 * j + i] = (WT)(int8_t)(q >> (8 * i));
+      }
+    }
+  }
+}
+
+// CTAS is the register budget (CTAs of 256 threads per SM): the host takes the
+// larger one unless the smaller saves passes over the resident clusters.
+// Loads ahead of the choice pay for float slices of one group per thread on the
+// larger budget only: n = 8192, 8 tasks on clusters of 8 6.06 -> 5.37 ms, 32 tasks
+// 7.23 -> 6.77; int8 rows (n = 6000, 20 tasks) 3.61 -> 4.09, many resident clusters
+// (n = 8192, 100 tasks, clusters of 16) 16.2 -> 19.7.
+template <typename WT, int NG, int CTAS>
+constexpr bool kAhead = sizeof(WT) == 4 && NG == 1 && CTAS == 2;
+
+template <typename WT, int NG, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) cluster_ascent_kernel(
     const ClusterGraph* __restrict__ graphs, const int* __restrict__ task_graph,
     const uint32_t* __restrict__ init_states, int words_pitch, int tasks, int spin,
     int flip_budget, uint32_t* __restrict__ best_states, double* __restrict__ best_values,
@@ -113,6 +149,12 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
     abort_flag = 0;
   }
   cl.sync();
+  // lane r's view of CTA r: this CTA's slot and the barrier of even exchanges
+  uint32_t rslot = 0, rbar = 0;
+  if (lane < C) {
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rslot) : "r"(tc::smem_u32(&slots[0][rank])), "r"(lane));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[0])), "r"(lane));
+  }
   uint32_t seq = 0;  // exchanges so far (over all tasks)
   const int clusters = gridDim.x / C;
   for (int task = blockIdx.x / C; task < tasks; task += clusters) {
@@ -178,33 +220,25 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
     int timeout = 0, failed = 0;
     int k = -1;
     GT coef = 0;
+    // the two runners-up of the last exchange, their row groups in flight
+    constexpr bool SPEC = kAhead<WT, NG, CTAS>;
+    const int vt = lo + 4 * (int)threadIdx.x;
+    int p1 = -1, p2 = -1, ahead = -1;
+    WT w1[4 * NG], w2[4 * NG];
+    unsigned long long sk = 0ull, gkey = 0ull;  // the last exchange: my lane's slot, the best
     double gk = 0.0;
     for (int f = 0;; ++f) {
       if (k >= 0) {
         // apply the previous flip (node k) to my fields
-        const WT* __restrict__ row = W + (size_t)k * G.ld;
         WT w[4 * NG];
+        if (SPEC && k == p1) {
 #pragma unroll
-        for (int j = 0; j < NG; ++j) {
-          const int v = lo + 4 * ((int)threadIdx.x + T * j);
-          if (v + 3 < n) {
-            if constexpr (sizeof(WT) == 4) {
-              const float4 t = __ldg(reinterpret_cast<const float4*>(row + v));
-              w[4 * j] = t.x;
-              w[4 * j + 1] = t.y;
-              w[4 * j + 2] = t.z;
-              w[4 * j + 3] = t.w;
-            } else {
-              const char4 t = __ldg(reinterpret_cast<const char4*>(row + v));
-              w[4 * j] = t.x;
-              w[4 * j + 1] = t.y;
-              w[4 * j + 2] = t.z;
-              w[4 * j + 3] = t.w;
-            }
-          } else {
+          for (int e = 0; e < 4 * NG; ++e) w[e] = w1[e];
+        } else if (SPEC && k == p2) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[4 * j + i] = (v + i < n) ? row[v + i] : (WT)0;
-          }
+          for (int e = 0; e < 4 * NG; ++e) w[e] = w2[e];
+        } else {
+          load_row<WT, NG>(W + (size_t)k * G.ld, vt, 4 * T, n, w);
         }
 #pragma unroll
         for (int j = 0; j < 4 * NG; ++j) y[j] += coef * (GT)w[j];
@@ -229,29 +263,28 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
       }
       // my best flip: float gain first, then the lowest node (nodes ascend)
       float bv = -INFINITY;
-      int bi = -1, bx = 0;
-      double bg = 0.0;
+      GT bg = 0;
+      int be = -1;  // element << 1 | bit
 #pragma unroll
-      for (int j = 0; j < NG; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int v = lo + 4 * ((int)threadIdx.x + T * j) + i;
-          if (v < hi) {
-            const int xv = (xm >> (4 * j + i)) & 1;
-            const double g = xv ? (double)y[4 * j + i] : -(double)y[4 * j + i];
-            const float gv = (float)g;
-            if (gv > bv) {  // strict: the lowest node keeps a tie
-              bv = gv;
-              bi = v;
-              bg = g;
-              bx = xv;
-            }
-          }
+      for (int e = 0; e < 4 * NG; ++e) {
+        const uint32_t xv = (xm >> e) & 1u;
+        GT g;
+        if constexpr (sizeof(WT) == 4) {
+          g = __hiloint2double(__double2hiint(y[e]) ^ (int)(xv ? 0u : 0x80000000u), __double2loint(y[e]));
+        } else {
+          g = xv ? y[e] : -y[e];
         }
-      const unsigned long long key = bi >= 0 ? flip_key(bv, bi, bx) : 0ull;
+        const float gv = (float)g;
+        const bool up = vt + 4 * T * (e >> 2) + (e & 3) < hi && gv > bv;  // strict: the lowest node keeps a tie
+        bv = up ? gv : bv;
+        bg = up ? g : bg;
+        be = up ? (int)(2 * e + xv) : be;
+      }
+      const unsigned long long key =
+          be >= 0 ? flip_key(bv, vt + 4 * T * (be >> 3) + ((be >> 1) & 3), be & 1) : 0ull;
       const unsigned long long wkey = warp_max_key(key);
       if (lane == 0) red_key[warp] = wkey;
-      if (key != 0ull && key == wkey) red_g[warp] = bg;
+      if (key != 0ull && key == wkey) red_g[warp] = (double)bg;
       const uint32_t par = seq & 1u, ph = (seq >> 1) & 1u;
       ++seq;
       if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(C * sizeof(Slot)));
@@ -266,22 +299,35 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
         // the next row is one of the C CTAs' candidates: pull this CTA's
         // candidate row into L2 while the exchange is in flight (a hint only;
         // a row is ld * sizeof(WT) bytes, 16-byte aligned, inside W)
-        if (lane == 0 && cb != 0ull && key_gain(cb) > 0.0f) {
-          const WT* cand = W + (size_t)key_node(cb) * G.ld;
+        if (lane == 0 && cb != 0ull && key_gain(cb) > 0.0f && key_node(cb) != ahead) {
+          ahead = key_node(cb);  // (one that stays the best is there already)
+          const WT* cand = W + (size_t)ahead * G.ld;
           asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(cand),
                        "r"((uint32_t)((size_t)G.ld * sizeof(WT)))
                        : "memory");
         }
         if (lane < C) {
-          uint32_t raddr, rbar;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                       : "=r"(raddr)
-                       : "r"(tc::smem_u32(&slots[par][rank])), "r"(lane));
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[par])), "r"(lane));
           asm volatile(
-              "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
-              "l"(cb), "l"(__double_as_longlong(cbg)), "r"(rbar)
+              "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(
+                  rslot + par * (uint32_t)sizeof(slots[0])),
+              "l"(cb), "l"(__double_as_longlong(cbg)), "r"(rbar + par * 8u)
               : "memory");
+        }
+      }
+      // While the exchange is in flight: the rows of the last exchange's second
+      // and third best, one of which is the next flip in half of the cases
+      // (measured on a dense Gaussian graph of 8192 nodes: 0.36 and 0.18).
+      if constexpr (SPEC) {
+        const unsigned long long s1 = sk == gkey ? 0ull : sk, k1 = warp_max_key(s1);
+        const unsigned long long k2 = warp_max_key(s1 == k1 ? 0ull : s1);
+        p1 = p2 = -1;
+        if (k1 != 0ull) {
+          p1 = key_node(k1);
+          load_row<WT, NG>(W + (size_t)p1 * G.ld, vt, 4 * T, n, w1);
+        }
+        if (k2 != 0ull) {
+          p2 = key_node(k2);
+          load_row<WT, NG>(W + (size_t)p2 * G.ld, vt, 4 * T, n, w2);
         }
       }
       if (!tc::mbar_wait_spin(&bar[par], ph)) {
@@ -289,9 +335,9 @@ __global__ void __launch_bounds__(256) cluster_ascent_kernel(
         break;
       }
       // the cluster's best (identical in every warp)
-      const unsigned long long sk = lane < C ? slots[par][lane].key : 0ull;
+      sk = lane < C ? slots[par][lane].key : 0ull;
       const double sg = lane < C ? slots[par][lane].g : 0.0;
-      const unsigned long long gkey = warp_max_key(sk);
+      gkey = warp_max_key(sk);
       if (rank == 0 && warp == 0) {  // the value is kept by warp 0 of CTA 0
         const uint32_t gsrc = __ballot_sync(0xFFFFFFFFu, sk == gkey);
         gk = __shfl_sync(0xFFFFFFFFu, sg, __ffs(gsrc) - 1);
@@ -394,19 +440,19 @@ extern "C" pqi_status pqi_cluster_ascent(const void* graphs, int num_graphs,
                                 as_stream(stream), &sf, &sf_pitch);
     if (r != PQI_OK) return r;
   }
-  auto launch = [&](auto kern) -> pqi_status {
+  // clusters resident at once (the occupancy query is cached per kernel and
+  // launch shape: it is slow on first use)
+  auto resident = [&](auto kern, int* out) -> pqi_status {
     PQI_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (cluster_size > 8)
       PQI_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    // as many clusters as fit at once; each loops over tasks (the occupancy
-    // query is cached per kernel and launch shape: it is slow on first use)
     struct FitEntry {
       const void* k;
       size_t smem;
       int T, cs, dev, fit;
     };
-    static FitEntry cache[32];
-    static int cached = 0;
+    static thread_local FitEntry cache[32];
+    static thread_local int cached = 0;
     int dev = 0;
     PQI_TRY(cudaGetDevice(&dev));
     int fit = 0;
@@ -423,25 +469,33 @@ extern "C" pqi_status pqi_cluster_ascent(const void* graphs, int num_graphs,
       set_error_text("cluster ascent: the cluster does not fit on the device");
       return PQI_EINVAL;
     }
-    const int clusters = std::max(1, std::min(tasks, fit));
-    cfg.gridDim = dim3(clusters * cluster_size);
+    *out = fit;
+    return PQI_OK;
+  };
+  // Two register budgets: a flip takes up to 12 % longer with the smaller one
+  // (n = 8192, clusters of 8), so it is for task counts where more resident
+  // clusters save passes over them (32 tasks on clusters of 16: 10.1 -> 7.0 ms).
+  auto launch = [&](auto fast, auto lean) -> pqi_status {
+    int ff = 0, fl = 0;
+    pqi_status r = resident(fast, &ff);
+    if (r == PQI_OK) r = resident(lean, &fl);
+    if (r != PQI_OK) return r;
+    const long long wf = (tasks + ff - 1) / ff, wl = (tasks + fl - 1) / fl;
+    const auto kern = wl * 9 < wf * 8 ? lean : fast;
+    cfg.gridDim = dim3(std::max(1, std::min(tasks, kern == lean ? fl : ff)) * cluster_size);
     PQI_TRY(cudaLaunchKernelEx(&cfg, kern, gd, task_graph, init_states, words_pitch, tasks,
                                is_spin_glass, flip_budget, best_states, best_values, flips_total,
                                status, target, reached, (const double*)sf, sf_pitch));
     return PQI_OK;
   };
-  pqi_status st;
-  if (i8) {
-    st = NG == 1   ? launch(cluster_ascent_kernel<int8_t, 1>)
-         : NG == 2 ? launch(cluster_ascent_kernel<int8_t, 2>)
-         : NG == 4 ? launch(cluster_ascent_kernel<int8_t, 4>)
-                   : launch(cluster_ascent_kernel<int8_t, 8>);
-  } else {
-    st = NG == 1   ? launch(cluster_ascent_kernel<float, 1>)
-         : NG == 2 ? launch(cluster_ascent_kernel<float, 2>)
-         : NG == 4 ? launch(cluster_ascent_kernel<float, 4>)
-                   : launch(cluster_ascent_kernel<float, 8>);
-  }
+  auto pick = [&](auto wt) -> pqi_status {
+    using WT = decltype(wt);
+    return NG == 1   ? launch(cluster_ascent_kernel<WT, 1, 2>, cluster_ascent_kernel<WT, 1, 4>)
+           : NG == 2 ? launch(cluster_ascent_kernel<WT, 2, 2>, cluster_ascent_kernel<WT, 2, 3>)
+           : NG == 4 ? launch(cluster_ascent_kernel<WT, 4, 1>, cluster_ascent_kernel<WT, 4, 2>)
+                     : launch(cluster_ascent_kernel<WT, 8, 1>, cluster_ascent_kernel<WT, 8, 1>);
+  };
+  const pqi_status st = i8 ? pick(int8_t{}) : pick(float{});
   if (st != PQI_OK) return st;
   PQI_LAUNCHED("cluster_ascent_kernel");
   if (sf) PQI_TRY(cudaFreeAsync(sf, as_stream(stream)));
