@@ -214,15 +214,18 @@ __global__ void __launch_bounds__(kGrayThreads) gray_kernel(
 // as few synchronisations as the size allows:
 //  * one warp (n <= 512): two redux steps, no barrier;
 //  * one CTA: each warp's best through shared memory, one barrier;
-//  * a cluster (CL): every warp sends its best to every CTA with st.async,
-//    counted on that CTA's mbarrier, and every warp waits for all of them and
-//    reduces them itself: one exchange, no CTA barrier. Two slot arrays and
-//    mbarriers alternate; a warp sends flip f + 2 only after all warps have
-//    read flip f (each sends f + 1 after that), so a slot is not overwritten
-//    while it is read.
-// While the row of the flipped node loads, the rows of new candidates - the next
-// flips are mostly among the warps' bests - are pulled into L2. Times: see pqi_single_descent.
-constexpr int DC_SLOTS = 256;  // warps of the largest launch: 16 CTAs x 512 threads
+//  * a cluster (CL): behind one CTA barrier warp 0 sends the CTA's best to every
+//    CTA with st.async, counted on that CTA's mbarrier; every warp waits for all
+//    of them and reduces them itself. (Every warp sending its own best saved the
+//    barrier, but the reduction of 64 arrivals took 10 to 20 % of a flip.) Two
+//    slot arrays and mbarriers alternate: a CTA sends flip f + 2 only after every
+//    CTA has sent f + 1, so all its warps have read f, and a slot is not
+//    overwritten while it is read.
+// During the exchange each warp pulls its best's row into L2 when it is a new
+// one: the next flips are mostly among the warps' bests. (Loading the last
+// exchange's runners-up into registers as well gained nothing below 12000 nodes
+// and cost 17 % at 4096, whose matrix stays in L2.) Times: see pqi_single_descent.
+constexpr int DC_SLOTS = 16;  // CTAs of a cluster, or warps of the one CTA, at most
 
 struct __align__(16) DescentBest {
   uint32_t hi;    // ordered float value (0: none selectable)
@@ -242,10 +245,6 @@ __device__ __forceinline__ DescentBest warp_best(const DescentBest& b) {
   return r;
 }
 
-__device__ __forceinline__ void better(DescentBest& b, const DescentBest& o) {
-  if (o.hi > b.hi || (o.hi == b.hi && o.lo > b.lo)) b = o;
-}
-
 template <typename WT, int NG, bool CL>
 __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp, int ld, int n,
                                                       uint32_t* __restrict__ theta, double* __restrict__ g64,
@@ -255,6 +254,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
   namespace cg = cooperative_groups;
   __shared__ DescentBest slots[2][DC_SLOTS];
   __shared__ __align__(8) uint64_t bar[2];
+  __shared__ DescentBest wbest[DC_SLOTS];  // this CTA's warps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = blockDim.x, nwarps = T >> 5;
   int C = 1, rank = 0;
   if constexpr (CL) {
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
     }
     cg::this_cluster().sync();
   }
-  const int nslots = C * nwarps;
+  const int nslots = CL ? C : nwarps;
   const int v0 = 4 * (rank * NG * T + (int)threadIdx.x);  // group j starts at v0 + 4 T j
   double g[4 * NG];
   uint32_t lo[4 * NG], xm = 0;
@@ -282,11 +282,15 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       lo[4 * j + i] = in ? (uint32_t)sel_key(0.0f, (uint64_t)(v + i), geo) : 0u;
     }
   }
-  const int slice = 4 * rank * NG * T;  // this CTA's first node
-  const uint32_t slice_bytes = slice < ld ? (uint32_t)(min(4 * NG * T, ld - slice) * (int)sizeof(WT)) : 0u;
   uint32_t seen = 0xFFFFFFFFu;
   double esum = 0.0;
   int cnt = 0, st = PQI_OK;
+  // lane r's view of CTA r: this CTA's slot and the barrier of even exchanges
+  uint32_t rslot = 0, rbar = 0;
+  if (CL && lane < C) {
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rslot) : "r"(tc::smem_u32(&slots[0][rank])), "r"(lane));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[0])), "r"(lane));
+  }
   for (int f = 0;; ++f) {
     // the thread's best, as floats (a -0 below a +0 does not matter here: only
     // values above 0 are taken); NaN compares false throughout
@@ -304,19 +308,27 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
     }
     DescentBest b{bl ? ord_f32(bv) : 0u, bl, be, 0u};
     b = warp_best(b);
+    const DescentBest own = b;
     const int par = f & 1;
     if constexpr (CL) {
-      if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(nslots * sizeof(DescentBest)));
-      if (lane < C) {
-        uint32_t raddr, rbar;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                     : "=r"(raddr)
-                     : "r"(tc::smem_u32(&slots[par][rank * nwarps + warp])), "r"(lane));
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rbar) : "r"(tc::smem_u32(&bar[par])), "r"(lane));
-        asm volatile(
-            "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(raddr),
-            "l"((uint64_t)b.lo << 32 | b.hi), "l"((uint64_t)b.node), "r"(rbar)
-            : "memory");
+      if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(C * sizeof(DescentBest)));
+      if (lane == 0) wbest[warp] = b;
+      __syncthreads();
+      if (warp == 0) {
+        b = warp_best(lane < nwarps ? wbest[lane] : DescentBest{0u, 0u, 0u, 0u});
+        if (lane < C)
+          asm volatile(
+              "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u64 [%0], {%1, %2}, [%3];" ::"r"(
+                  rslot + par * (uint32_t)sizeof(slots[0])),
+              "l"((uint64_t)b.lo << 32 | b.hi), "l"((uint64_t)b.node), "r"(rbar + par * 8u)
+              : "memory");
+      }
+      // a new best of this warp: its row into L2 (a hint)
+      if (lane == 0 && own.hi > 0x80000000u && own.node >> 1 != seen) {
+        seen = own.node >> 1;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Wp + (size_t)seen * ld),
+                     "r"((uint32_t)(ld * (int)sizeof(WT)))
+                     : "memory");
       }
       if (!tc::mbar_wait_spin(&bar[par], (uint32_t)(f >> 1) & 1u)) {
         st = PQI_ECUDA;  // a peer stopped sending
@@ -327,9 +339,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       __syncthreads();
     }
     if (CL || nwarps > 1) {
-      DescentBest c{0u, 0u, 0u, 0u};
-      for (int q = lane; q < nslots; q += 32) better(c, slots[par][q]);
-      b = warp_best(c);
+      b = warp_best(lane < nslots ? slots[par][lane] : DescentBest{0u, 0u, 0u, 0u});
     }
     const float val = b.lo ? unord_f32(b.hi) : -INFINITY;
     if (!(val > 0.0f)) break;
@@ -358,20 +368,6 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[4 * j + i] = (WT)0;
-      }
-    }
-    if constexpr (CL) {
-      // This CTA's slice of the rows of new candidates (a warp's best that was
-      // not its best before), into L2: a hint. Warp w looks after warp w of
-      // every CTA, one per lane.
-      if (lane < C) {
-        const uint32_t node = slots[par][lane * nwarps + warp].node >> 1;
-        if (node != seen && slice_bytes > 0u) {
-          seen = node;
-          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Wp + (size_t)node * ld + slice),
-                       "r"(slice_bytes)
-                       : "memory");
-        }
       }
     }
 #pragma unroll
@@ -516,8 +512,8 @@ pqi_status pqi_single_descent(const pqi_weights* w, uint32_t* theta, double* gai
   // Threads of 4 NG nodes: one warp up to 128 nodes, one CTA up to kDescentCta,
   // else a cluster. Microseconds per flip, one CTA with the gains in shared
   // memory and the tie rule's divisions per node -> now: complete float graphs
-  // of 300 nodes 2.8 -> 1.1, 1000 3.9 -> 0.90, 2048 4.5 -> 0.95, 4096 5.6 -> 1.10,
-  // 8192 8.2 -> 1.35 (a whole descent 38.4 -> 6.3 ms), 16384 13.9 -> 1.52.
+  // of 300 nodes 2.8 -> 1.06, 1000 3.9 -> 0.85, 2048 4.5 -> 0.90, 4096 5.6 -> 0.97,
+  // 8192 8.2 -> 1.13 (a whole descent 38.4 -> 5.3 ms), 16384 13.9 -> 1.20.
   const int groups = (n + 3) / 4;
   int C = 1, T = 32, NG = 1;
   auto shape = [&](int c, int tmax) {
