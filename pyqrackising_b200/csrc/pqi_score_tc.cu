@@ -531,7 +531,9 @@ __global__ void __launch_bounds__(FUSED ? FTHREADS : PTHREADS, 1)
       __syncwarp();
       if (lane == 0) {  // accumulator a may be overwritten
         if (PAIR && rank == 1) {
-          mbar_arrive_remote0(&acce_bar[a]);  // the even CTA issues the MMAs
+          // to the even CTA, which issues the MMAs (the loads are complete, so
+          // nothing but the signal leaves this CTA)
+          mbar_signal_remote0(&acce_bar[a]);
         } else {
           mbar_arrive(&acce_bar[a]);
         }

@@ -238,12 +238,13 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
-// Arrive on the barrier at the same offset in CTA 0 of the cluster.
-__device__ __forceinline__ void mbar_arrive_remote0(uint64_t* bar) {
+// Arrive on the barrier at the same offset in CTA 0 of the cluster, releasing at
+// CTA scope: for signals about data that stay in the arriving CTA (its shared or
+// tensor memory). A release to the cluster holds the thread for 1,500 cycles.
+__device__ __forceinline__ void mbar_signal_remote0(uint64_t* bar) {
   uint32_t remote;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(smem_u32(bar)));
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote)
-               : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
 
 }  // namespace tc
