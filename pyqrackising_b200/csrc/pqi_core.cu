@@ -73,7 +73,7 @@ struct PrepStats {
 // partial per tile (0 below the diagonal). Reads W once, the next pair's loads in
 // flight, one barrier per pair; classification counts are reduced at the end. A
 // block per tile that read both tiles and reduced everything through shared
-// memory took 425 us at n = 8192, this 123 (268 MB).
+// memory took 425 us at n = 8192, this 110 (268 MB, bound by issue).
 __global__ void __launch_bounds__(256) prep_scan_kernel(const float* __restrict__ W, int n, int tb, PrepStats* st,
                                                         double* __restrict__ partial) {
   __shared__ float tT[2][32][33];
@@ -82,15 +82,12 @@ __global__ void __launch_bounds__(256) prep_scan_kernel(const float* __restrict_
   const long long pairs = (long long)tb * (tb + 1) / 2;
   unsigned int nf = 0, ni = 0, as = 0;
   float mx = 0.0f;
-  auto tile_of = [&](long long q, int* bi, int* bj) {  // q = J (J + 1) / 2 + I
-    long long J = (long long)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
-    while (J * (J + 1) / 2 > q) --J;
-    while ((J + 1) * (J + 2) / 2 <= q) ++J;
-    *bj = (int)J;
-    *bi = (int)(q - J * (J + 1) / 2);
-  };
   float a[4], b[4];  // W[i][j] and, to be transposed, W[j][i]
-  int bi = 0, bj = 0, last = -1;
+  // pair p = J (J + 1) / 2 + I, advanced column by column
+  int bi = (int)blockIdx.x, bj = 0, last = -1;
+  auto settle = [&]() {
+    while (bi > bj) bi -= ++bj;
+  };
   auto load = [&]() {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -119,7 +116,7 @@ __global__ void __launch_bounds__(256) prep_scan_kernel(const float* __restrict_
   };
   long long p = blockIdx.x;
   if (p < pairs) {
-    tile_of(p, &bi, &bj);
+    settle();
     load();
   }
   int par = 0;
@@ -132,7 +129,8 @@ __global__ void __launch_bounds__(256) prep_scan_kernel(const float* __restrict_
     }
     const int I = bi, J = bj;
     if (p + gridDim.x < pairs) {
-      tile_of(p + gridDim.x, &bi, &bj);
+      bi += (int)gridDim.x;
+      settle();
       load();
     }
     __syncthreads();
