@@ -189,8 +189,9 @@ __global__ void apply_flip_kernel(const long long* __restrict__ ptr, const int* 
   if (l >= 0) block_flip<uint32_t>(g, theta, ptr, col, val, l);
 }
 
-// Gray search, one CTA per seed (grid-stride), the dense gray kernel's walk
-// (kernels.cl:894-978 semantics; see pqi_gray.cu) with CSR flips. The 64-bit
+// Gray search, one CTA per seed (grid-stride): the dense gray kernel's schedule
+// (kernels.cl:894-978 semantics; see pqi_gray.cu), 32 positions tested per step,
+// with CSR flips. The 64-bit
 // state words sit in shared memory, the seed's gains in g_all + block * n.
 __global__ void __launch_bounds__(256) gray_kernel(
     const long long* __restrict__ ptr, const int* __restrict__ col, const float* __restrict__ val,
