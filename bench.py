@@ -16,7 +16,8 @@ and selected with its tie rule. One step = one batch.
   buffered so the next step's copy overlaps this step's scoring), scores it
   through the C ABI and reads the (best value, index) pair back.
 * roofline: the scoring GEMM (the integer ops of the node tiles on and below the
-  diagonal, 2*B*n^2 * (T+1)/(2T) for T tiles of 256 nodes) against the int8 tensor rate, taken as twice the measured dense bf16 rate.
+  diagonal, 2*B*n^2 * (T+1)/(2T) for T tiles of 256 nodes) against the int8
+  tensor rate, taken as twice the measured dense bf16 rate.
 * cpu_baseline: the reference's CPU scoring path (numba: compute_cut_diff_between
   per candidate under prange, maxcut_tfim.py:77-136), restated in
   oracle/numba_port.py and pinned to the reference's own values, on all host

@@ -412,8 +412,8 @@ static size_t gray_smem_bytes(int n, size_t gain_bytes) {
 static constexpr size_t kMaxGraySmem = 208 * 1024;
 
 // Largest graph that descends in one CTA (512 threads of four nodes): at 2048
-// nodes 0.95 us per flip against 1.22 with a cluster, at 4096 (two groups per
-// thread) 1.32 against 1.17.
+// nodes 0.90 us per flip against 1.01 with a cluster, at 4096 (two groups per
+// thread) 1.32 against 0.97.
 constexpr int kDescentCta = 2048;  // 512 * 4 at most
 
 // CTAs of a descent's cluster: 16 where the device can place them.
