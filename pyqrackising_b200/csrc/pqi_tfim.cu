@@ -560,9 +560,10 @@ struct __align__(16) SparseEntry {
 };
 
 // Control words: some weight is -1; some weight is not in {0, +1, -1}; nonzero
-// weights; the largest number of them in a row.
+// weights; the largest number of them in a row; some row of few has an entry
+// whose mirror image is zero, so a column may be fuller than every row.
 struct SampleCtl {
-  unsigned minus, other, count, degree;
+  unsigned minus, other, count, degree, lopsided;
 };
 
 // Tables of W's rows, a warp per row through shared memory:
@@ -586,9 +587,9 @@ __global__ void __launch_bounds__(1024) tfim_rows_kernel(const float* __restrict
   auto factor = [&](float w) {
     return w == 0.0f ? 1.0 : w == 1.0f ? rep1 : w == -1.0f ? repm1 : repulsion_factor(lnb, w);
   };
-  if (threadIdx.x == 0) sc = SampleCtl{0u, 0u, 0u, 0u};
+  if (threadIdx.x == 0) sc = SampleCtl{0u, 0u, 0u, 0u, 0u};
   __syncthreads();
-  unsigned minus_any = 0, other = 0, count = 0, degree = 0;
+  unsigned minus_any = 0, other = 0, count = 0, degree = 0, lopsided = 0;
   for (int r = blockIdx.x * wpb + wib; r < n; r += gridDim.x * wpb) {
     const float* row = W + (size_t)r * n;
     int at = 0;
@@ -599,6 +600,8 @@ __global__ void __launch_bounds__(1024) tfim_rows_kernel(const float* __restrict
       if (slots && w != 0.0f) {
         const int e = at + __popc(nz & ((1u << lane) - 1u));
         if (e < SP_DEG) slots[(size_t)r * SP_DEG + e] = SparseEntry{factor(w), v, w == -1.0f};
+        // (only as many as a row may have for the codes: a dozen loads per row)
+        if (e < SP_CODE_DEG && __ldg(W + (size_t)v * n + r) == 0.0f) lopsided = 1;
       }
       at += __popc(nz);
     }
@@ -632,6 +635,7 @@ __global__ void __launch_bounds__(1024) tfim_rows_kernel(const float* __restrict
   if (other) atomicOr(&sc.other, 1u);
   if (count) atomicAdd(&sc.count, count);
   if (lane == 0) atomicMax(&sc.degree, degree);
+  if (lopsided) atomicOr(&sc.lopsided, 1u);
   __syncthreads();
   if (threadIdx.x == 0) {
     if (gridDim.x == 1) {
@@ -641,15 +645,19 @@ __global__ void __launch_bounds__(1024) tfim_rows_kernel(const float* __restrict
       if (sc.other) atomicOr(&ctl->other, 1u);
       atomicAdd(&ctl->count, sc.count);
       atomicMax(&ctl->degree, sc.degree);
+      if (sc.lopsided) atomicOr(&ctl->lopsided, 1u);
     }
   }
 }
 
 // Which form the weights call for. codes / lists: the sparse forms are there
-// (chosen by n in tfim_sample_impl).
+// (chosen by n in tfim_sample_impl). A node's factors come by its column, so its
+// code holds them all only where the columns are no fuller than the rows: the
+// pattern of the weights must be its own mirror image (the caller's W need not
+// be symmetric).
 enum SampleForm { SF_BITS, SF_TABLE, SF_LISTS, SF_CODES };
 __device__ __forceinline__ SampleForm sample_form(const SampleCtl& c, bool codes, bool lists) {
-  if (codes && !c.other && c.degree <= SP_CODE_DEG) return SF_CODES;
+  if (codes && !c.other && !c.lopsided && c.degree <= SP_CODE_DEG) return SF_CODES;
   if (lists && c.degree <= SP_DEG) return SF_LISTS;
   return c.other ? SF_TABLE : SF_BITS;
 }
@@ -874,7 +882,7 @@ __global__ void __launch_bounds__(64, sr_blocks(C, TABLE))
 // sums their groups anew, so a pick costs O(degree) groups instead of n weights.
 // The chain of a pick (a row load, the groups' sums, two scans) is latency, so
 // what counts is how many shots an SM holds: float64 weights leave 13 at n =
-// 2048. Where every weight is +-1 and no row has more than SP_CODE_DEG (CODES),
+// 2048. Where every weight is +-1 and no row or column has more than SP_CODE_DEG (CODES),
 // a weight is one of 2^(SP_CODE_DEG + 1) products of factors in the order of the
 // picks, so a byte names it - a leading 1, then a bit per factor; 0 for a picked
 // node - and a table holds the products, multiplied in that order.

@@ -62,3 +62,26 @@ def test_forms_draw_the_same_candidates(kind, n):
         a = _draw(dg, cum, shots, base, 11, full)
         b = _draw(dg, cum, shots, base, 11, small)
         assert torch.equal(a, b), (shots, base)
+
+
+@pytest.mark.parametrize("n,kind", [(300, "column"), (1500, "column"), (300, "ring"), (1100, "ring")])
+def test_weights_need_not_be_symmetric(n, kind):
+    """A bare W: every row has at most three +-1 entries, one column has one in
+    every row ("column"), or the entries of a ring run one way ("ring")."""
+    rng = np.random.default_rng(n)
+    i = np.arange(n)
+    W = np.zeros((n, n), dtype=np.float32)
+    for k in (1, 5):
+        W[i, (i + k) % n] = rng.choice(np.array([-1.0, 1.0], dtype=np.float32), n)
+    if kind == "column":
+        W[:, 7] = 1.0
+    np.fill_diagonal(W, 0.0)
+    sym = D.DeviceGraph(_weights("ring1", n, rng))
+    _, _, cum = MT.hamming_cdf(sym, 2, 8.0, 8.0)
+    full = torch.empty(_lib.load().pqi_tfim_sample_workspace_bytes(n), dtype=torch.uint8, device=sym.device)
+    small = torch.empty(1024, dtype=torch.uint8, device=sym.device)
+    sym.W = torch.from_numpy(W).to(sym.device)
+    for base in (5.0, 0.5):
+        a = _draw(sym, cum, 512, base, 11, full)
+        b = _draw(sym, cum, 512, base, 11, small)
+        assert torch.equal(a, b), base
