@@ -468,6 +468,9 @@ __global__ void tfim_sample_kernel(const float* __restrict__ W, int n,
             }
             run += __shfl_sync(0xFFFFFFFFu, w, 31);
           }
+          // the lanes' prefixes are summed in different orders, so one without
+          // nodes may be above p by a rounding: as if none were
+          if (picked >= n) picked = 0;
         }
         node = picked;
       }
@@ -839,16 +842,19 @@ __global__ void __launch_bounds__(64, sr_blocks(C, TABLE))
         }
       }
       // bit_pick (util:711-724): p = sum(weights) * u, the first node whose
-      // running sum is above p (node 0 when none is)
+      // running sum is above p; node 0 when none is, or when the roundings of
+      // sums in different orders lead to a slot past the last node
       const double loc = tree_sum<0, NG, NG>(sum);
       const double incl = warp_scan(loc);
       const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
       const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
+      node = n;
       if (hit) {
         const int owner = __ffs(hit) - 1;
         slot = pick_node<0, C, C>(w, sum, p - (incl - loc), owner, lane);
         node = owner * C + slot;
-      } else {
+      }
+      if (node >= n) {
         if (lane == 0) w[0] = 0.0;
         slot = node = 0;
       }
@@ -1003,7 +1009,7 @@ __global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
       const double incl = warp_scan(loc);
       const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
       const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
-      node = 0;  // no prefix above p
+      node = n;
       if (hit) {
         const int owner = __ffs(hit) - 1;
         double q = p - (incl - loc);
@@ -1017,6 +1023,7 @@ __global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
         const unsigned h2 = __ballot_sync(0xFFFFFFFFu, q < warp_scan(weight(32 * g + lane)));
         node = 32 * g + (h2 ? __ffs(h2) - 1 : 0);
       }
+      if (node >= n) node = 0;  // no prefix above p, or led past the last node by a rounding
       if (lane == 0) {
         if constexpr (CODES) {
           code[node] = 0;
