@@ -269,12 +269,14 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
   }
   const int nslots = CL ? C : nwarps;
   const int v0 = 4 * (rank * NG * T + (int)threadIdx.x);  // group j starts at v0 + 4 T j
+  typedef typename std::conditional<NG <= 8, uint32_t, uint64_t>::type Mask;  // a bit per node
   double g[4 * NG];
-  uint32_t lo[4 * NG], xm = 0;
+  uint32_t lo[4 * NG];
+  Mask xm = 0;
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
     const int v = v0 + 4 * T * j;
-    if (v < ((n + 31) & ~31)) xm |= ((theta[v >> 5] >> (v & 31)) & 15u) << (4 * j);
+    if (v < ((n + 31) & ~31)) xm |= (Mask)((theta[v >> 5] >> (v & 31)) & 15u) << (4 * j);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool in = v + i < n;
@@ -303,7 +305,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       if (lo[e] != 0u && (v > bv || (v == bv && lo[e] > bl))) {
         bv = v;
         bl = lo[e];
-        be = (uint32_t)(v0 + 4 * T * (e >> 2) + (e & 3)) << 1 | ((xm >> e) & 1u);
+        be = (uint32_t)(v0 + 4 * T * (e >> 2) + (e & 3)) << 1 | (uint32_t)((xm >> e) & 1u);
       }
     }
     DescentBest b{bl ? ord_f32(bv) : 0u, bl, be, 0u};
@@ -376,9 +378,9 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       const double w2 = 2.0 * (double)w[e];
       if (v == k) {
         g[e] = -g[e];
-        xm ^= 1u << e;
+        xm ^= (Mask)1 << e;
       } else {
-        g[e] += ((xm >> e) & 1u) == xk ? -w2 : w2;
+        g[e] += (uint32_t)((xm >> e) & 1u) == xk ? -w2 : w2;
       }
     }
   }
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
 #pragma unroll
   for (int j = 0; j < NG; ++j) {
     const int v = v0 + 4 * T * j;
-    uint32_t wd = ((xm >> (4 * j)) & 15u) << (4 * (lane & 7));
+    uint32_t wd = ((uint32_t)(xm >> (4 * j)) & 15u) << (4 * (lane & 7));
     wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 1);
     wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 2);
     wd |= __shfl_xor_sync(0xFFFFFFFFu, wd, 4);
@@ -561,7 +563,7 @@ pqi_status pqi_single_descent(const pqi_weights* w, uint32_t* theta, double* gai
            : NG == 2 ? launch(descent_kernel<WT, 2, true>, wp)
            : NG == 4 ? launch(descent_kernel<WT, 4, true>, wp)
            : NG == 8 ? launch(descent_kernel<WT, 8, true>, wp)
-                     : launch(descent_kernel<WT, 16, true>, wp);  // (past the dense matrices that fit)
+                     : launch(descent_kernel<WT, 16, true>, wp);  // (int8 past 262144 nodes)
   };
   const pqi_status rc = w->kind == PQI_W_I8 ? pick((const int8_t*)w->W_i8) : pick((const float*)w->W_f32z);
   if (rc != PQI_OK) return rc;
