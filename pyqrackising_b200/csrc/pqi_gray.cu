@@ -220,7 +220,12 @@ __global__ void __launch_bounds__(kGrayThreads) gray_kernel(
 //    barrier, but the reduction of 64 arrivals took 10 to 20 % of a flip.) Two
 //    slot arrays and mbarriers alternate: a CTA sends flip f + 2 only after every
 //    CTA has sent f + 1, so all its warps have read f, and a slot is not
-//    overwritten while it is read.
+//    overwritten while it is read. A wait that runs out, which one warp or lane
+//    may see alone, raises the CTA's flag of that exchange; the warp goes on with
+//    what its slots hold (an older node of the graph, or none), every warp passes
+//    one more CTA barrier, the next flip's or the one behind the loop, and reads
+//    the flag behind it, so the CTA leaves together and the others follow by
+//    their own waits.
 // During the exchange each warp pulls its best's row into L2 when it is a new
 // one: the next flips are mostly among the warps' bests. (Loading the last
 // exchange's runners-up into registers as well gained nothing below 12000 nodes
@@ -255,6 +260,8 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
   __shared__ DescentBest slots[2][DC_SLOTS];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ DescentBest wbest[DC_SLOTS];  // this CTA's warps
+  __shared__ int wait_failed[2];           // by parity of the exchange
+  __shared__ int any_failed;               // in rank 0: some CTA's wait ran out
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = blockDim.x, nwarps = T >> 5;
   int C = 1, rank = 0;
   if constexpr (CL) {
@@ -264,7 +271,9 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       tc::mbar_init(&bar[0], 1);
       tc::mbar_init(&bar[1], 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      wait_failed[0] = wait_failed[1] = any_failed = 0;
     }
+    if (threadIdx.x < 2 * DC_SLOTS) slots[threadIdx.x & 1][threadIdx.x >> 1] = DescentBest{0u, 0u, 0u, 0u};
     cg::this_cluster().sync();
   }
   const int nslots = CL ? C : nwarps;
@@ -286,7 +295,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
   }
   uint32_t seen = 0xFFFFFFFFu;
   double esum = 0.0;
-  int cnt = 0, st = PQI_OK;
+  int cnt = 0, st = PQI_OK, failed = 0;
   // lane r's view of CTA r: this CTA's slot and the barrier of even exchanges
   uint32_t rslot = 0, rbar = 0;
   if (CL && lane < C) {
@@ -316,6 +325,7 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       if (threadIdx.x == 0) tc::mbar_expect_tx(&bar[par], (uint32_t)(C * sizeof(DescentBest)));
       if (lane == 0) wbest[warp] = b;
       __syncthreads();
+      failed = wait_failed[par ^ 1];  // another warp's last wait ran out
       if (warp == 0) {
         b = warp_best(lane < nwarps ? wbest[lane] : DescentBest{0u, 0u, 0u, 0u});
         if (lane < C)
@@ -332,10 +342,8 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
                      "r"((uint32_t)(ld * (int)sizeof(WT)))
                      : "memory");
       }
-      if (!tc::mbar_wait_spin(&bar[par], (uint32_t)(f >> 1) & 1u)) {
-        st = PQI_ECUDA;  // a peer stopped sending
-        break;
-      }
+      if (failed) break;
+      if (!tc::mbar_wait_spin(&bar[par], (uint32_t)(f >> 1) & 1u)) wait_failed[par] = 1;
     } else if (nwarps > 1) {
       if (lane == 0) slots[par][warp] = b;
       __syncthreads();
@@ -344,9 +352,13 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
       b = warp_best(lane < nslots ? slots[par][lane] : DescentBest{0u, 0u, 0u, 0u});
     }
     const float val = b.lo ? unord_f32(b.hi) : -INFINITY;
-    if (!(val > 0.0f)) break;
-    if (cnt >= max_flips) {
-      st = PQI_ETIMEOUT;
+    const bool none = !(val > 0.0f);
+    if (none || cnt >= max_flips) {
+      st = none ? PQI_OK : PQI_ETIMEOUT;
+      if constexpr (CL) {
+        __syncthreads();  // (the one that warps which go on pass in their next flip)
+        failed = wait_failed[par];
+      }
       break;
     }
     esum += (double)val;
@@ -397,13 +409,16 @@ __global__ void __launch_bounds__(512) descent_kernel(const WT* __restrict__ Wp,
     for (int i = 0; i < 4; ++i)
       if (v + i < n) g64[v + i] = g[4 * j + i];
   }
+  if constexpr (CL) {
+    if (failed && threadIdx.x == 0) *cg::this_cluster().map_shared_rank(&any_failed, 0) = 1;
+    cg::this_cluster().sync();  // (and no CTA leaves while another may still send to it)
+    if (any_failed) st = PQI_ECUDA;
+  }
   if (rank == 0 && threadIdx.x == 0) {
     *energy_sum = esum;
     *flips = cnt;
     *status = st;
   }
-  // (no CTA leaves while another may still send to it)
-  if constexpr (CL) cg::this_cluster().sync();
 }
 
 static size_t gray_smem_bytes(int n, size_t gain_bytes) {

@@ -1,6 +1,7 @@
 """How the warps of a cluster leave a loop of exchanges when a bounded wait runs out
-in some of them only: the barriers of pqi_cluster.cu's flip loop, restated as
-coroutines and run in random orders. Every warp must reach every barrier, whichever
+in some of them only: the barriers of the flip loops of the cluster ascent
+(pqi_cluster.cu) and the descent (pqi_gray.cu), restated as coroutines and run in
+random orders. Every warp must reach every barrier, whichever
 waits fail, and the whole cluster must come to one verdict."""
 
 import random
