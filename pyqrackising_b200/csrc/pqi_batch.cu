@@ -1375,6 +1375,7 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         }
       }
     }
+    tm_wait_st();  // the last pass's fields: the columns go to the next task, or back
     if (t == 0) {
       best_values[task] = best;
       atomicAdd(flips_total, nflips);

@@ -44,3 +44,21 @@ def test_bound_keeps_the_selection(kind, sizes):
     assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
     # (the starting value sums x_v y_v in another order; the gains added are equal)
     assert torch.all((got[0] - want[0]).abs() <= 1e-10 * (want[0].abs() + max(sizes) * 1e-38))
+
+
+def test_tasks_that_follow_one_another_in_the_same_columns():
+    """Several tasks per CTA, of two sizes: each starts from its own fields, whatever
+    the one before still had on the way."""
+    sizes = (4097, 6000)
+    bs = BatchedSearch([D.DeviceGraph(_matrix("wide", n, n)) for n in sizes], row_lists=False)
+    tg = (np.arange(1500, dtype=np.int32) // 2) % 2
+    words = bs.random_states(tg, 6)
+    args = dict(rounds=1, kick=3, seed=12, flip_budget=25)
+    got = bs.run(tg, words, True, **args)
+    _lib.call("pqi_batch_set_tmem_fields", 0)
+    try:
+        want = bs.run(tg, words, True, **args)
+    finally:
+        _lib.call("pqi_batch_set_tmem_fields", 1)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    assert torch.all((got[0] - want[0]).abs() <= 1e-10 * (want[0].abs() + 1.0))
