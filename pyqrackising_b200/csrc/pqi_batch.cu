@@ -1119,7 +1119,7 @@ __device__ __forceinline__ void tm_pass(const TmCtx& c, int k, int xk, uint32_t 
     // overlap (a branch per group of four ran them one after the other, 70
     // cycles per node). Nodes at and past n update fields that nothing reads.
     if (UPD) {
-      if (!tc::mbar_wait_spin(&bars[q], (phase >> q) & 1u)) *s_fail = 1;  // this chunk of the row
+      if (!tc::mbar_wait_spin(&bars[q], (phase >> q) & 1u)) s_fail[par] = 1;  // this chunk of the row
       float4 s4[4];
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) s4[jj] = *reinterpret_cast<const float4*>(c.stage + v0 + 512 * jj);
@@ -1201,7 +1201,7 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
   __shared__ unsigned long long red_key[2][4];
   __shared__ double red_g[2][4];
   __shared__ double s_yk[2];
-  __shared__ int s_fail;
+  __shared__ int s_fail[2];  // by parity of the pass
   __shared__ __align__(8) uint64_t row_bar[J / 4];  // one per 2048 nodes of the row
   __shared__ uint32_t s_tmem;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -1217,7 +1217,7 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (t == 0) {
-    s_fail = 0;
+    s_fail[0] = s_fail[1] = 0;
     for (int q = 0; q < J / 4; ++q) tc::mbar_init(&row_bar[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1302,7 +1302,8 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
     // has finished reading the previous row: the pass before ended on a CTA
     // barrier). The pass's threads wait for the copies themselves (bounded); a
     // wait that runs out anywhere raises a flag that all read behind the pass's
-    // barrier, so it stops the task everywhere.
+    // barrier, so it stops the task everywhere. (Each pass has the other flag than
+    // the one before, which a slow warp may still have to read.)
     float rw[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // the references' weights to k
     auto fetch = [&](int k) {
       const float* row = c.W + (size_t)k * c.ld;
@@ -1320,7 +1321,7 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         }
       }
     };
-    tm_pass<false, false, J>(c, -1, 0, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel, &gflip);
+    tm_pass<false, false, J>(c, -1, 0, xm, refs, rw, row_bar, phase, s_fail, red_key, red_g, s_yk, par, &key, &gsel, &gflip);
     par ^= 1;
     for (int r = 0; r <= rounds && !failed; ++r) {
       for (int f = 0;; ++f) {
@@ -1333,15 +1334,15 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         const int xk = (int)(key & 1ull);
         fetch(k);
         val += scale * gsel;
-        tm_pass<true, false, J>(c, k, xk, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel,
+        tm_pass<true, false, J>(c, k, xk, xm, refs, rw, row_bar, phase, s_fail, red_key, red_g, s_yk, par, &key, &gsel,
                                 &gflip);
-        par ^= 1;
         phase ^= used;
         ++nflips;
-        if (s_fail) {
+        if (s_fail[par]) {
           failed = true;
           break;
         }
+        par ^= 1;
       }
       if (failed) break;
       if (val > best) {
@@ -1363,16 +1364,16 @@ __global__ void __launch_bounds__(TM_BT, TmShape<J>::CTAS) batch_search_tmem_ker
         __syncthreads();  // everyone has read bit and kicked set before they change
         if (t == 0) kicked[pick >> 5] |= 1u << (pick & 31);
         fetch(pick);
-        tm_pass<true, true, J>(c, pick, xp, xm, refs, rw, row_bar, phase, &s_fail, red_key, red_g, s_yk, par, &key, &gsel,
+        tm_pass<true, true, J>(c, pick, xp, xm, refs, rw, row_bar, phase, s_fail, red_key, red_g, s_yk, par, &key, &gsel,
                                &gflip);
-        par ^= 1;
         phase ^= used;
         val += scale * gflip;  // float64 gain of the kicked node
         ++nflips;
-        if (s_fail) {
+        if (s_fail[par]) {
           failed = true;
           break;
         }
+        par ^= 1;
       }
     }
     tm_wait_st();  // the last pass's fields: the columns go to the next task, or back

@@ -1,25 +1,27 @@
 """How the warps of a cluster leave a loop of exchanges when a bounded wait runs out
 in some of them only: the barriers of the flip loops of the cluster ascent
 (pqi_cluster.cu) and the descent (pqi_gray.cu), restated as coroutines and run in
-random orders. Every warp must reach every barrier, whichever
-waits fail, and the whole cluster must come to one verdict."""
+random orders. Every warp must reach every barrier, whichever waits fail, and the
+whole cluster must come to one verdict. (The passes of the tensor-memory search,
+pqi_batch.cu, alternate their flags for the reason of the last case.)"""
 
 import random
 
 import pytest
 
 
-def _warp(cta, warp, flips, S, flags, report, uniform, rng, inside=None):
+def _warp(cta, warp, flips, S, flags, report, uniform, rng, inside=None, flip=1):
     """One warp's barriers. uniform: the verdict is taken behind a CTA barrier;
     else a warp whose wait runs out leaves by itself. inside: a flip before which
-    the cluster meets (a barrier inside the loop)."""
+    the cluster meets (a barrier inside the loop). flip: flags alternate between
+    exchanges (0: one flag for all)."""
     f, failed = 0, 0
     while True:
         if f == inside:
             yield "cluster", "inside"
         yield "cta", 0
         yield "pause", 0  # (a slow warp reads the flag late)
-        failed = flags[cta][(f & 1) ^ 1]
+        failed = flags[cta][(f & flip) ^ flip]
         if warp == 0:
             S[f].add(cta)
         if uniform and failed:
@@ -27,7 +29,7 @@ def _warp(cta, warp, flips, S, flags, report, uniform, rng, inside=None):
         ok = yield "wait", f
         end = f == flips - 1  # every warp whose wait succeeded reads that no flip is left
         if not ok:
-            flags[cta][f & 1] = 1
+            flags[cta][f & flip] = 1
             end = rng.random() < 0.5  # (what the slots held)
         if not uniform:
             if end or not ok:
@@ -36,7 +38,7 @@ def _warp(cta, warp, flips, S, flags, report, uniform, rng, inside=None):
         elif end:
             yield "cta", 0
             yield "pause", 0
-            failed = flags[cta][f & 1]
+            failed = flags[cta][f & flip]
             break
         f += 1
     if failed:
@@ -45,10 +47,10 @@ def _warp(cta, warp, flips, S, flags, report, uniform, rng, inside=None):
     return bool(report)
 
 
-def _run(seed, uniform, ctas=3, warps=3, flips=3, chance=0.2, inside=None):
+def _run(seed, uniform, ctas=3, warps=3, flips=3, chance=0.2, inside=None, flip=1):
     rng = random.Random(seed)
     S, report, flags = [set() for _ in range(flips + 2)], set(), [[0, 0] for _ in range(ctas)]
-    gens = {(c, w): _warp(c, w, flips, S, flags, report, uniform, rng, inside) for c in range(ctas) for w in range(warps)}
+    gens = {(c, w): _warp(c, w, flips, S, flags, report, uniform, rng, inside, flip) for c in range(ctas) for w in range(warps)}
     at = {k: next(g) for k, g in gens.items()}  # what each warp stands at
     done = {}
 
@@ -103,3 +105,7 @@ def test_warps_that_leave_by_themselves_would_hang():
 
 def test_a_cluster_barrier_inside_the_loop_would_not_match():
     assert any(_run(seed, True, inside=2) is None for seed in range(200))
+
+
+def test_one_flag_for_all_exchanges_would_be_read_too_late():
+    assert any(_run(seed, True, flip=0) is None for seed in range(600))
