@@ -978,7 +978,9 @@ __global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
           // could lengthen a full code: left as it is)
           if (c && c < SP_TABLE / 2 && col != node) code[col] = (uint8_t)(2 * c + e.minus);
         } else {
-          if (col != node) w[col] *= e.factor;
+          // (the node itself where the slot is its diagonal, not an empty one: 0
+          // stays 0, unless the factor is not finite)
+          if (col != node || e.factor != 1.0) w[col] *= e.factor;
         }
       }
       __syncwarp();

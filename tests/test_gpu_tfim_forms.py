@@ -85,3 +85,22 @@ def test_weights_need_not_be_symmetric(n, kind):
         a = _draw(sym, cum, 512, base, 11, full)
         b = _draw(sym, cum, 512, base, 11, small)
         assert torch.equal(a, b), base
+
+
+@pytest.mark.parametrize("n", [300, 1100, 2048])
+def test_diagonal_with_an_infinite_factor(n):
+    """base^(-w) overflows for a diagonal weight of -500: the picked node's weight,
+    zero until then, is NaN from there on in every form."""
+    rng = np.random.default_rng(n)
+    W = _weights("mix3", n, rng)
+    i = rng.choice(n, n // 8, replace=False)
+    W[i, i] = -500.0
+    sym = D.DeviceGraph(_weights("ring1", n, rng))
+    _, _, cum = MT.hamming_cdf(sym, 2, 8.0, 8.0)
+    full = torch.empty(_lib.load().pqi_tfim_sample_workspace_bytes(n), dtype=torch.uint8, device=sym.device)
+    small = torch.empty(1024, dtype=torch.uint8, device=sym.device)
+    sym.W = torch.from_numpy(W).to(sym.device)
+    for base in (5.0, 0.2):
+        a = _draw(sym, cum, 256, base, 11, full)
+        b = _draw(sym, cum, 256, base, 11, small)
+        assert torch.equal(a, b), base
