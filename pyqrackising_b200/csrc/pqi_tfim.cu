@@ -848,13 +848,15 @@ __global__ void __launch_bounds__(64, sr_blocks(C, TABLE))
       const double incl = warp_scan(loc);
       const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
       const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
-      node = n;
       if (hit) {
         const int owner = __ffs(hit) - 1;
         slot = pick_node<0, C, C>(w, sum, p - (incl - loc), owner, lane);
         node = owner * C + slot;
-      }
-      if (node >= n) {
+        if (node >= n) {
+          if (lane == 0) w[0] = 0.0;
+          slot = node = 0;
+        }
+      } else {
         if (lane == 0) w[0] = 0.0;
         slot = node = 0;
       }
@@ -1011,7 +1013,7 @@ __global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
       const double incl = warp_scan(loc);
       const double p = __shfl_sync(0xFFFFFFFFu, incl, 31) * __shfl_sync(0xFFFFFFFFu, us, j & 31);
       const unsigned hit = __ballot_sync(0xFFFFFFFFu, p < incl);
-      node = n;
+      node = 0;  // no prefix above p
       if (hit) {
         const int owner = __ffs(hit) - 1;
         double q = p - (incl - loc);
@@ -1024,8 +1026,8 @@ __global__ void __launch_bounds__(32 * sp_warps(CODES), CODES ? 12 : 16)
         q = __shfl_sync(0xFFFFFFFFu, q, owner);
         const unsigned h2 = __ballot_sync(0xFFFFFFFFu, q < warp_scan(weight(32 * g + lane)));
         node = 32 * g + (h2 ? __ffs(h2) - 1 : 0);
+        node = node < n ? node : 0;  // (led past the last node by a rounding)
       }
-      if (node >= n) node = 0;  // no prefix above p, or led past the last node by a rounding
       if (lane == 0) {
         if constexpr (CODES) {
           code[node] = 0;
