@@ -553,7 +553,10 @@ pqi_status pqi_tfim_cdf(const double* J_eff, const unsigned int* degrees, int n,
                         double anneal_t, double anneal_h, const double* thresholds, double* cum,
                         void* workspace, size_t workspace_bytes, void* stream);
 
-/* Workspace bytes pqi_tfim_sample needs for n nodes (large n only). */
+/* Workspace bytes for pqi_tfim_sample on n nodes. Up to 2048 nodes with W it holds
+ * the row tables of the register and sparse forms; with less (or none) the
+ * shared-memory form draws the same candidates several times slower. Beyond 4960
+ * nodes it holds the weights themselves and is required. */
 size_t pqi_tfim_sample_workspace_bytes(int n);
 
 /* Draw `shots` candidates as packed bits (shots x ceil(n/32) words): shot s
@@ -568,9 +571,10 @@ pqi_status pqi_tfim_sample(const float* W, int n, const double* cum, double repu
 
 /* pqi_tfim_sample with the nonzero entries of W's rows as lists (row r's
  * columns adj_col[adj_ptr[r] .. adj_ptr[r+1]) ascending, values adj_val, from
- * pqi_tfim_adj_count / pqi_tfim_adj_fill): a repulsion update
- * (maxcut_tfim.py:37-45) walks the picked node's list instead of scanning its
- * row. The same multiplications in the same order: the same draws, bit for bit. */
+ * pqi_tfim_adj_count / pqi_tfim_adj_fill): above 2048 nodes, or without W, a
+ * repulsion update (maxcut_tfim.py:37-45) walks the picked node's list instead of
+ * scanning its row; up to 2048 nodes with W (and the workspace) the lists are not
+ * read. The same multiplications in the same order: the same draws, bit for bit. */
 pqi_status pqi_tfim_sample_adj(const float* W, int n, const long long* adj_ptr, const int* adj_col,
                                const float* adj_val, const double* cum, double repulsion_base,
                                uint64_t seed, uint64_t round, int shots, uint32_t* theta_out,

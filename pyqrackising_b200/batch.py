@@ -105,9 +105,9 @@ class BatchedSearch:
         the float64 objective and the returned value is float64-exact. The
         ranking can differ from float64 fields' where gains agree to float32
         rounding. "auto" (default): "f64" while its fields fit in shared
-        memory (up to 24576 nodes; it is also the faster form there: SK
-        n = 8192 flip updates run at 0.50 of HBM bandwidth against 0.35 with
-        "f32"), "f32" beyond.
+        memory (up to 24576 nodes; it is also the faster form where they fit
+        in tensor memory, up to 16384: SK n = 8192 flip updates run at 0.83
+        of HBM bandwidth against 0.36 with "f32"), "f32" beyond.
         Integer graphs are exact either way.
 
         `out` = (best_states, best_values, flips, status) device buffers to

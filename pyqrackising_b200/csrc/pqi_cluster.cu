@@ -13,8 +13,8 @@
 //      k toggles its bit) and folds the new gains g_v = x_v y_v into a local
 //      argmax: float gain first, then the lowest node (a 64-bit key);
 //      (branch-free; with it and a row prefetch only for candidates that change,
-//      n = 6000 int8, 20 tasks on clusters of 8, went from 4.47 to 3.71 ms and
-//      n = 8192 float, 8 tasks, from 6.98 to 6.06, 5.38 with the loads of kAhead);
+//      n = 6000 int8, 20 tasks on clusters of 8, went from 4.47 to 3.61 ms and
+//      n = 8192 float, 8 tasks, from 6.98 to 6.06, 5.37 with the loads of kAhead);
 //   2. warp maxima (two 32-bit redux steps) meet in shared memory behind the
 //      flip's one CTA barrier; warp 0 reduces them and its lanes 0..C-1 write the
 //      CTA's best (key, exact gain) into slot [rank] of every CTA with st.async,
@@ -35,8 +35,9 @@
 // alternate, so that none is raised while a slow warp has yet to read the one
 // before.) The other CTAs, which it no longer sends to, follow by their own waits;
 // the cluster's barriers stand outside the loop, the same number for every CTA. So
-// the flip budget and the bounded waits end every loop. (With the verdict in the
-// maximum, or by a reducing barrier, flips took 3 to 7 % longer.)
+// the flip budget and the bounded waits end every loop. (It costs 1.6 % of a float
+// flip: n = 8192, 8 tasks on clusters of 8 5.37 -> 5.46 ms, and none of an int8 one;
+// with the verdict in the maximum, or by a reducing barrier, 4 to 8 %.)
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -189,10 +189,10 @@ __global__ void apply_flip_kernel(const long long* __restrict__ ptr, const int* 
   if (l >= 0) block_flip<uint32_t>(g, theta, ptr, col, val, l);
 }
 
-// Gray search, one CTA per seed (grid-stride): the dense gray kernel's schedule
-// (kernels.cl:894-978 semantics; see pqi_gray.cu), 32 positions tested per step,
-// with CSR flips. The 64-bit
-// state words sit in shared memory, the seed's gains in g_all + block * n.
+// Gray search, one CTA per seed (grid-stride): the schedule of kernels.cl:894-978,
+// 32 of its positions tested per step (the dense kernel of pqi_gray.cu visits the
+// same positions by words of positive gains), with CSR flips. The 64-bit state
+// words sit in shared memory, the seed's gains in g_all + block * n.
 __global__ void __launch_bounds__(256) gray_kernel(
     const long long* __restrict__ ptr, const int* __restrict__ col, const float* __restrict__ val,
     int n, const uint64_t* __restrict__ theta64, const double* __restrict__ base_g, int spin,

@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kGrayThreads) gray_kernel(
 // serial, so the kernel is bound by its latency; a thread keeps the gains, bits
 // and tie priorities of 4 NG nodes in registers and the selection goes through
 // as few synchronisations as the size allows:
-//  * one warp (n <= 512): two redux steps, no barrier;
-//  * one CTA: each warp's best through shared memory, one barrier;
+//  * one warp (n <= 128): two redux steps, no barrier;
+//  * one CTA (to kDescentCta): each warp's best through shared memory, one barrier;
 //  * a cluster (CL): behind one CTA barrier warp 0 sends the CTA's best to every
 //    CTA with st.async, counted on that CTA's mbarrier; every warp waits for all
 //    of them and reduces them itself. (Every warp sending its own best saved the
@@ -430,7 +430,7 @@ static constexpr size_t kMaxGraySmem = 208 * 1024;
 
 // Largest graph that descends in one CTA (512 threads of four nodes): at 2048
 // nodes 0.90 us per flip against 1.01 with a cluster, at 4096 (two groups per
-// thread) 1.32 against 0.97.
+// thread) 1.32 against 0.96.
 constexpr int kDescentCta = 2048;  // 512 * 4 at most
 
 // CTAs of a descent's cluster: 16 where the device can place them.
@@ -529,8 +529,8 @@ pqi_status pqi_single_descent(const pqi_weights* w, uint32_t* theta, double* gai
   // Threads of 4 NG nodes: one warp up to 128 nodes, one CTA up to kDescentCta,
   // else a cluster. Microseconds per flip, one CTA with the gains in shared
   // memory and the tie rule's divisions per node -> now: complete float graphs
-  // of 300 nodes 2.8 -> 1.06, 1000 3.9 -> 0.85, 2048 4.5 -> 0.90, 4096 5.6 -> 0.97,
-  // 8192 8.2 -> 1.13 (a whole descent 38.4 -> 5.3 ms), 16384 13.9 -> 1.20.
+  // of 300 nodes 2.8 -> 1.06, 1000 3.9 -> 0.85, 2048 4.5 -> 0.90, 4096 5.6 -> 0.96,
+  // 8192 8.2 -> 1.12 (a whole descent 38.4 -> 5.3 ms), 16384 13.9 -> 1.20.
   const int groups = (n + 3) / 4;
   int C = 1, T = 32, NG = 1;
   auto shape = [&](int c, int tmax) {

@@ -528,8 +528,8 @@ pqi_status pqi_mpnn_gemm(int transA, int transB, int M, int N, int K, float alph
   dim3 grid((N + mp::TN - 1) / mp::TN, (M + mp::TM - 1) / mp::TM);
   // Below two 64 x 64 tiles per SM the warp tiles are faster at every shape of
   // the network (n 128 to 16384). Per gradient (K = n = 1024, 128 x 64 outputs)
-  // 120 us -> 16 us; a training example (forward and backward) n = 1024 887 ->
-  // 400 us, of which 330 is the host's launches, n = 4096 2818 -> 809, n = 16384
+  // 120 us -> 16 us; a training example (forward and backward) n = 1024 897 ->
+  // 350 us, of which 330 is the host's launches, n = 4096 2818 -> 809, n = 16384
   // 13.0 -> 3.1 ms.
   if ((long long)grid.x * grid.y < mp::SM_MAX_TILES) {
     const dim3 small((N + mp::SM_TN - 1) / mp::SM_TN, (M + mp::SM_TM - 1) / mp::SM_TM);
