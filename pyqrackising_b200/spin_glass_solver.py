@@ -132,6 +132,12 @@ def local_search(dg, theta, is_spin_glass: bool, gray_iterations: int, gray_seed
             row = tout[bx * 2 * dg.n64 : bx * 2 * dg.n64 + dg.n32].clone()
             if n & 31:
                 row[-1] &= (1 << (n & 31)) - 1  # bits >= n are padding (the reference unpacks bits < n)
+            # A walk that comes back to where it began (or flips a whole component) changes
+            # nothing, but its float gains can sum to a rounding above 0, and would do so for
+            # ever (200 of 35,700 searches on 8192 nodes). The re-scored objective depends on
+            # the state alone: it has to rise. (Integer gains sum exactly.)
+            if not dg.is_integer and not bool(dg.rescore(row)[0] > dg.rescore(words)[0]):
+                break
             words[: dg.n32] = row
             _, g64 = dg.gains(words)
             max_energy += e
